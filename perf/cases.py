@@ -249,3 +249,88 @@ def tolerance(case):
         # eight, 1.6e-2 / 7.6e-2 after 28
         return dict(rel=1.6e-2, max=1e-1) if case["layers"] <= 2 else dict(rel=3e-2, max=3e-1)
     return TOLERANCE[case["op"]]
+
+
+# -------------------------------------------------------------------- exact ---
+def _norm64(x, weight=None):
+    y = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6)
+    return y if weight is None else y * weight.double()
+
+
+def _rotate64(x, cos, sin):
+    """x [B, heads, D], tables [B, D]: the two halves of a head are the rotated pairs."""
+    a, b = x.chunk(2, -1)
+    return x * cos.double()[:, None] + torch.cat([-b, a], -1) * sin.double()[:, None]
+
+
+def _attend64(q, K, V, lens):
+    """q [B, H, D]; K(b) and V(b) give a row's [NKV, S, D]; the first lens[b] keys count."""
+    rows = []
+    for b, n in enumerate(lens):
+        k, v = K(b)[:, :n].double(), V(b)[:, :n].double()
+        p = (q[b].view(k.shape[0], -1, k.shape[2]) @ k.transpose(1, 2) * k.shape[2] ** -0.5).softmax(-1)
+        rows.append((p @ v).reshape(q.shape[1], -1))
+    return torch.stack(rows)
+
+
+def _swiglu64(x2, weight, Wg, Wu, Wd):
+    xn = _norm64(x2, weight)
+    return x2 + (torch.nn.functional.silu(xn @ Wg.double().T) * (xn @ Wu.double().T)) @ Wd.double().T
+
+
+def _layer64(x, L, sh, lens, cos=None, sin=None, pages=None):
+    """One layer in 64 bits; returns its output and the caches as they stand afterwards."""
+    B, D, NKV = x.shape[0], sh.head_dim, sh.num_kv_heads
+    qkv = _norm64(x, L.get("input_norm_w")) @ L["Wqkv"].double().T
+    q, k, v = (t.reshape(B, -1, D) for t in qkv.split([sh.q_rows, sh.kv_rows, sh.kv_rows], -1))
+    q, k = _norm64(q, L.get("q_norm_w")), _norm64(k, L.get("k_norm_w"))
+    if cos is not None:
+        at = torch.tensor(lens, device=x.device) - 1
+        q, k = _rotate64(q, cos[at], sin[at]), _rotate64(k, cos[at], sin[at])
+    Kc, Vc = L["K_cache"].double(), L["V_cache"].double()
+    if pages is None:
+        row = lambda t: lambda b: t[b]  # noqa: E731
+    else:
+        row = lambda t: lambda b: t[pages[b].long()].transpose(0, 1).reshape(NKV, -1, D)  # noqa: E731
+    for b, n in enumerate(lens):
+        slot = (b, n - 1) if pages is None else (int(pages[b, (n - 1) // Kc.shape[2]]), (n - 1) % Kc.shape[2])
+        Kc[slot[0], :, slot[1]], Vc[slot[0], :, slot[1]] = k[b], v[b]
+    x2 = x + _attend64(q, row(Kc), row(Vc), lens).reshape(B, -1) @ L["Wo"].double().T
+    Wg, Wu = L["Wgu"].chunk(2)
+    return _swiglu64(x2, L.get("post_norm_w"), Wg, Wu, L["Wd"]), Kc, Vc
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs, computed by torch in 64 bits with no rounding in between."""
+    state = prepare(case, seed)
+    args, op = state["args"], case["op"]
+    if op == "gemv":
+        return args[1].double() @ args[0].double()
+    if op == "rmsnorm":
+        return _norm64(args[0].double(), args[1] if case["dtype"] == "bf16" else None)
+    if op == "qk_rope":
+        q, k, v, qw, kw, cos, sin, Kc, Vc = args
+        at = [n - 1 for n in _lengths(case, seed, 1)]
+        q, k = (_rotate64(_norm64(t.double(), w), cos[at], sin[at]) for t, w in ((q, qw), (k, kw)))
+        Kc, Vc = Kc.double(), Vc.double()
+        for b, slot in enumerate(at):
+            Kc[b, :, slot], Vc[b, :, slot] = k[b], v[b].double()
+        return (q, k), Kc, Vc
+    if op == "attn":
+        Q, K, V = args
+        lens = _lengths(case, seed, case["min_len"]) if case["min_len"] else [case["S"]] * case["B"]
+        return _attend64(Q[:, :, 0].double(), lambda b: K[b], lambda b: V[b], lens)[:, :, None]
+    if op == "ffn":
+        attn, residual, Wo, weight, Wg, Wu, Wd = args
+        return _swiglu64(residual.double() + attn.double() @ Wo.double().T, weight, Wg, Wu, Wd)
+    sh, B, S = SHAPES[case["model"]], case["B"], case["S"]
+    if op == "layer":
+        names = ("K_cache", "V_cache", "Wqkv", "Wo", "Wgu", "Wd")
+        return _layer64(args[0].double(), dict(zip(names, args[1:])), sh, [S] * B)
+    hidden, layers, cos, sin = args
+    lens = _lengths(case, seed, max(1, S // 8)) if case["ragged"] else [S] * B
+    x, caches = hidden.double(), []
+    for L in layers:
+        x, *kv = _layer64(x, L, sh, lens, cos, sin, state["kw"].get("page_table"))
+        caches += kv
+    return (x, *caches)
