@@ -143,22 +143,10 @@ static size_t round256(size_t v) { return (v + 255) / 256 * 256; }
 // the counters that must start at zero.
 struct LayerWorkspace {
     void* attn;
-    void* tc;  // tensor-core path: split counters (zero between calls) and partial tiles; null at batch 1
     bf16 *qkv, *attn_out, *x2, *h, *xn;
     void* mega;  // batch 1: barrier counters and slice records of the single-kernel layer (zero before first use)
     size_t total;
 };
-
-// Largest tensor-core workspace any projection of a layer with these sizes needs.
-static size_t layer_tc_bytes(int B, int H, int I, int rows_qkv) {
-    if (B < 2) return 0;
-    size_t m = gemm_tc_workspace_bytes(B, rows_qkv, false);
-    size_t v = gemm_tc_workspace_bytes(B, H, false);
-    if (v > m) m = v;
-    v = gemm_tc_workspace_bytes(B, I, true);
-    if (v > m) m = v;
-    return m;
-}
 
 static LayerWorkspace carve_layer_ws(void* base, int B, int S, int H, int I, int NH, int NKV, int D) {
     LayerWorkspace w;
@@ -170,8 +158,6 @@ static LayerWorkspace carve_layer_ws(void* base, int B, int S, int H, int I, int
         return r;
     };
     w.attn = take(attn_workspace_bytes(B, NH, NKV, S, D));
-    const size_t tc_bytes = layer_tc_bytes(B, H, I, (NH + 2 * NKV) * D);
-    w.tc = tc_bytes ? take(tc_bytes) : nullptr;
     w.qkv = reinterpret_cast<bf16*>(take((size_t)B * (NH + 2 * NKV) * D * 2));
     w.attn_out = reinterpret_cast<bf16*>(take((size_t)B * NH * D * 2));
     w.x2 = reinterpret_cast<bf16*>(take((size_t)B * H * 2));
@@ -183,7 +169,6 @@ static LayerWorkspace carve_layer_ws(void* base, int B, int S, int H, int I, int
 }
 
 struct FfnWorkspace {
-    void* tc;
     bf16 *x2, *h, *xn;
     size_t total;
 };
@@ -197,8 +182,6 @@ static FfnWorkspace carve_ffn_ws(void* base, int B, int H, int I) {
         off += round256(bytes);
         return r;
     };
-    const size_t tc_bytes = layer_tc_bytes(B, H, I, H);
-    w.tc = tc_bytes ? take(tc_bytes) : nullptr;
     w.x2 = reinterpret_cast<bf16*>(take((size_t)B * H * 2));
     w.h = reinterpret_cast<bf16*>(take((size_t)B * I * 2));
     w.xn = reinterpret_cast<bf16*>(take((size_t)B * H * 2));
@@ -233,10 +216,9 @@ static PrefetchList one_plan(const PrefetchPlan& a) {
 
 // o_proj (+residual or fp32 partial), gate/up + SwiGLU, down (+residual or fp32 partial)
 static cudaError_t launch_o_proj(const bf16* attn, const bf16* Wo, int B, int H, int Q, const bf16* residual, void* out,
-                                 bool f32_partial, cudaStream_t stream, const PrefetchList& next = kNoPrefetch,
-                                 void* tc = nullptr) {
+                                 bool f32_partial, cudaStream_t stream, const PrefetchList& next = kNoPrefetch) {
     GemvArgs g;
-    g.tc_workspace = tc;
+    g.allow_tc = B >= 2;
     g.W0 = Wo, g.ldw = Q, g.N = H, g.K = Q, g.B = B;
     g.x = attn, g.ldx = Q;
     g.prologue = PRO_NONE;
@@ -250,9 +232,9 @@ static cudaError_t launch_o_proj(const bf16* attn, const bf16* Wo, int B, int H,
 
 static cudaError_t launch_gate_up(const bf16* x, const float* x_add, bf16* x_sum_out, const bf16* norm_w, const bf16* Wg,
                                   const bf16* Wu, int B, int H, int I, float eps, bf16* h, bf16* xn_scratch,
-                                  cudaStream_t stream, const PrefetchList& next = kNoPrefetch, void* tc = nullptr) {
+                                  cudaStream_t stream, const PrefetchList& next = kNoPrefetch) {
     GemvArgs g;
-    g.tc_workspace = tc;
+    g.allow_tc = B >= 2;
     g.W0 = Wg, g.W1 = Wu, g.ldw = H, g.N = I, g.K = H, g.B = B;
     g.x = x, g.ldx = H;
     g.x_add = x_add, g.ldadd = H, g.x_sum_out = x_sum_out, g.ldsum = H;
@@ -267,10 +249,9 @@ static cudaError_t launch_gate_up(const bf16* x, const float* x_add, bf16* x_sum
 }
 
 static cudaError_t launch_down(const bf16* h, const bf16* Wd, int B, int H, int I, const bf16* residual, void* out,
-                               bool f32_partial, cudaStream_t stream, const PrefetchList& next = kNoPrefetch,
-                               void* tc = nullptr) {
+                               bool f32_partial, cudaStream_t stream, const PrefetchList& next = kNoPrefetch) {
     GemvArgs g;
-    g.tc_workspace = tc;
+    g.allow_tc = B >= 2;
     g.W0 = Wd, g.ldw = I, g.N = H, g.K = I, g.B = B;
     g.x = h, g.ldx = I;
     g.prologue = PRO_NONE;
@@ -312,7 +293,7 @@ static cudaError_t launch_qkv_and_attention(const bf16* hidden, bf16* Kc, bf16* 
     g.eps = eps, g.prologue = PRO_RMSNORM, g.epilogue = EPI_STORE;
     g.out = w.qkv, g.ldout = rows;
     g.xn_scratch = w.xn;
-    g.tc_workspace = w.tc;
+    g.allow_tc = B >= 2;
     g.trace_id = 1;
     // while the projection drains, start pulling the KV cache (if it is small enough to sit in L2)
     const size_t kv_bytes = (size_t)B * NKV * S * D * 2;
@@ -413,16 +394,15 @@ int ezb_gemv_bf16(const void* x, const void* W, void* y, int N, int K, ezb_strea
 }
 
 size_t ezb_gemv_workspace_bytes(int B, int N, int K) {
-    (void)K;
-    if (B < 2 || N < 1) return 256;
-    return gemm_tc_workspace_bytes(B, N, false);  // split counters and partial tiles of the tensor-core path
+    (void)B, (void)N, (void)K;
+    return 256;  // no kernel behind this entry needs scratch memory in device global memory
 }
 
 int ezb_gemv_batched_bf16(const void* X, const void* W, void* Y, void* workspace, size_t workspace_bytes, int B, int N, int K,
                           ezb_stream_t stream) {
     EZB_REQUIRE(X && W && Y, "null pointer");
     EZB_REQUIRE(N >= 1 && K >= 1 && B >= 1, "B, N and K must be positive");
-    if (B >= 2 && (!workspace || workspace_bytes < gemm_tc_workspace_bytes(B, N, false))) {
+    if (B >= 2 && (!workspace || workspace_bytes < ezb_gemv_workspace_bytes(B, N, K))) {
         set_last_message("workspace missing or smaller than ezb_gemv_workspace_bytes()");
         return EZB_ERR_WORKSPACE;
     }
@@ -433,7 +413,7 @@ int ezb_gemv_batched_bf16(const void* X, const void* W, void* Y, void* workspace
     g.W0 = static_cast<const bf16*>(W), g.ldw = K, g.N = N, g.K = K, g.B = B;
     g.x = static_cast<const bf16*>(X), g.ldx = K;
     g.out = Y, g.ldout = N;
-    g.tc_workspace = B >= 2 ? workspace : nullptr;
+    g.allow_tc = B >= 2;
     chain_begin();
     EZB_CUDA_TRY(launch_gemv(g, stream));
     return EZB_OK;
@@ -569,11 +549,11 @@ int ezb_o_proj_ffn(const void* attn, const void* residual, const void* Wo, const
     const int pf_kb = tuning(EZB_TUNE_L2_PREFETCH_KB);
     EZB_CUDA_TRY(launch_o_proj(static_cast<const bf16*>(attn), static_cast<const bf16*>(Wo), B, H, Q,
                                static_cast<const bf16*>(residual), w.x2, false, stream,
-                               one_plan(next_rows(static_cast<const bf16*>(Wg), static_cast<const bf16*>(Wu), I, H, pf_kb)), w.tc));
+                               one_plan(next_rows(static_cast<const bf16*>(Wg), static_cast<const bf16*>(Wu), I, H, pf_kb))));
     EZB_CUDA_TRY(launch_gate_up(w.x2, nullptr, nullptr, static_cast<const bf16*>(post_norm_w), static_cast<const bf16*>(Wg),
                                 static_cast<const bf16*>(Wu), B, H, I, eps, w.h, w.xn, stream,
-                                one_plan(next_rows(static_cast<const bf16*>(Wd), nullptr, H, I, pf_kb)), w.tc));
-    EZB_CUDA_TRY(launch_down(w.h, static_cast<const bf16*>(Wd), B, H, I, w.x2, out, false, stream, kNoPrefetch, w.tc));
+                                one_plan(next_rows(static_cast<const bf16*>(Wd), nullptr, H, I, pf_kb))));
+    EZB_CUDA_TRY(launch_down(w.h, static_cast<const bf16*>(Wd), B, H, I, w.x2, out, false, stream, kNoPrefetch));
     return EZB_OK;
 }
 
@@ -615,11 +595,11 @@ static int run_layer(const bf16* hid, bf16* Kc, bf16* Vc, const bf16* Wqkv, cons
     EZB_CUDA_TRY(launch_qkv_and_attention(hid, Kc, Vc, Wqkv, w, B, S, H, NH, NKV, D, eps, stream, Wo,
                                           pf_attn_kb > 0 ? &gu_head : nullptr, ex));
     EZB_CUDA_TRY(launch_o_proj(w.attn_out, Wo, B, H, NH * D, hid, w.x2, false, stream,
-                               one_plan(next_rows(wgu, wgu + (size_t)I * H, I, H, pf_kb, pf_attn_kb > 0 ? pf_attn_kb : 0)), w.tc));
+                               one_plan(next_rows(wgu, wgu + (size_t)I * H, I, H, pf_kb, pf_attn_kb > 0 ? pf_attn_kb : 0))));
     EZB_CUDA_TRY(launch_gate_up(w.x2, nullptr, nullptr, ex.post_norm_w, wgu, wgu + (size_t)I * H, B, H, I, eps, w.h, w.xn, stream,
-                                one_plan(next_rows(Wd, nullptr, H, I, pf_kb)), w.tc));
+                                one_plan(next_rows(Wd, nullptr, H, I, pf_kb))));
     const PrefetchList after = ex.next_Wqkv ? one_plan(next_rows(ex.next_Wqkv, nullptr, (NH + 2 * NKV) * D, H, pf_kb)) : kNoPrefetch;
-    EZB_CUDA_TRY(launch_down(w.h, Wd, B, H, I, w.x2, out, false, stream, after, w.tc));
+    EZB_CUDA_TRY(launch_down(w.h, Wd, B, H, I, w.x2, out, false, stream, after));
     return EZB_OK;
 }
 
@@ -717,7 +697,7 @@ int ezb_qwen3_decode_layer_tp_attn(const void* hidden, void* K_cache, void* V_ca
                                           static_cast<bf16*>(V_cache), static_cast<const bf16*>(Wqkv_local), w, B, S, H,
                                           NH_local, NKV_local, D, eps, stream, static_cast<const bf16*>(Wo_local)));
     EZB_CUDA_TRY(launch_o_proj(w.attn_out, static_cast<const bf16*>(Wo_local), B, H, NH_local * D, nullptr, partial_o, true,
-                               stream, kNoPrefetch, w.tc));
+                               stream, kNoPrefetch));
     return EZB_OK;
 }
 
@@ -738,9 +718,9 @@ int ezb_qwen3_decode_layer_tp_ffn(const void* hidden, const float* summed_o, con
     chain_begin();
     EZB_CUDA_TRY(launch_gate_up(static_cast<const bf16*>(hidden), summed_o, static_cast<bf16*>(x2), nullptr, wgu,
                                 wgu + (size_t)I_local * H, B, H, I_local, eps, w.h, w.xn, stream,
-                                one_plan(next_rows(static_cast<const bf16*>(Wd_local), nullptr, H, I_local, tuning(EZB_TUNE_L2_PREFETCH_KB))), w.tc));
+                                one_plan(next_rows(static_cast<const bf16*>(Wd_local), nullptr, H, I_local, tuning(EZB_TUNE_L2_PREFETCH_KB)))));
     EZB_CUDA_TRY(launch_down(w.h, static_cast<const bf16*>(Wd_local), B, H, I_local, nullptr, partial_d, true, stream,
-                             kNoPrefetch, w.tc));
+                             kNoPrefetch));
     return EZB_OK;
 }
 
@@ -905,7 +885,7 @@ static int check_tp_fused_shape(int B, int H, int I_local, int NH_local, int NKV
     // every projection must run a kernel that knows the exchange: the small-batch kernel, or (batch >= 2)
     // the tensor-core kernel with the row kernel in front
     auto covered = [&](int K, int N, bool pair) {
-        return gemv_small_batch_eligible(B, K) || (tuning(EZB_TUNE_TC) != 0 && gemm_tc_supported(B, K) && gemm_tc_fits(N, pair));
+        return gemv_small_batch_eligible(B, K) || (tuning(EZB_TUNE_TC) != 0 && gemm_tc_supported(B, K));
     };
     EZB_REQUIRE_SHAPE(covered(H, (NH_local + 2 * NKV_local) * D, false) && covered(NH_local * D, H, false) &&
                           covered(H, I_local, true) && covered(I_local, H, false),
@@ -928,7 +908,7 @@ static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_
     const bf16* hid = gather_prev ? layer_in : x_prev;
     {   // QKV projection (norm prologue; gathers the previous layer's second sum when there is one)
         GemvArgs g;
-        g.tc_workspace = w.tc, g.xn_scratch = w.xn;
+        g.allow_tc = B >= 2, g.xn_scratch = w.xn;
         g.W0 = Wqkv, g.ldw = H, g.N = rows, g.K = H, g.B = B;
         g.x = x_prev, g.ldx = H;
         g.norm_w = ex.input_norm_w;
@@ -960,7 +940,7 @@ static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_
     }
     {   // o_proj: partial -> inbox 0 of every rank; also opens the next epoch of inbox 1
         GemvArgs g;
-        g.tc_workspace = w.tc, g.xn_scratch = w.xn;
+        g.allow_tc = B >= 2, g.xn_scratch = w.xn;
         g.W0 = Wo, g.ldw = Q, g.N = H, g.K = Q, g.B = B;
         g.x = w.attn_out, g.ldx = Q;
         g.epilogue = EPI_PUSH_F32, g.ldout = H;
@@ -971,7 +951,7 @@ static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_
     }
     {   // gate/up: x2 = layer input + sum(inbox 0), norm, SwiGLU
         GemvArgs g;
-        g.tc_workspace = w.tc, g.xn_scratch = w.xn;
+        g.allow_tc = B >= 2, g.xn_scratch = w.xn;
         g.W0 = wgu, g.W1 = wgu + (size_t)I_local * H, g.ldw = H, g.N = I_local, g.K = H, g.B = B;
         g.x = hid, g.ldx = H;
         g.x_sum_out = x2_out, g.ldsum = H;
@@ -985,7 +965,7 @@ static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_
     }
     {   // down: partial -> inbox 1 of every rank; opens the next epoch of inbox 0
         GemvArgs g;
-        g.tc_workspace = w.tc, g.xn_scratch = w.xn;
+        g.allow_tc = B >= 2, g.xn_scratch = w.xn;
         g.W0 = Wd, g.ldw = I_local, g.N = H, g.K = I_local, g.B = B;
         g.x = w.h, g.ldx = I_local;
         g.epilogue = EPI_PUSH_F32, g.ldout = H;

@@ -60,8 +60,8 @@ static constexpr long long kWaitLimitCycles = 2000000000LL;
 // read it.  Pull (EZB_TUNE_TP_PULL): the producer writes slot `rank` of its OWN buffer only and
 // consumers poll slot w of rank w's buffer with peer loads.  Measured on two GPUs (us per layer,
 // Qwen3-8B batch 32 KV 4096 | Qwen3-32B batch 64 KV 8192): NCCL all-reduce between the parts 162 | 345,
-// push 168 | 408, pull 200 | 433 - with the stream-K split only the 32-40 CTAs that finish a tile store,
-// 32-64 KB each, which takes them 16-22 us; at batch <= 8 (every CTA stores a few values) push is the fast one.
+// push 168 | 408, pull 200 | 433 - measured with a tensor-core kernel in which only the 32-40 CTAs that finished a tile
+// stored, 32-64 KB each (16-22 us); at batch <= 8 (every CTA stores a few values) push is the fast one.
 // ---------------------------------------------------------------------------
 struct TpLink {
     int world;  // 0: no fused exchange
@@ -483,21 +483,27 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // launched this way calls pdl_wait() before it reads or writes anything the
 // predecessor touches.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                       Args... args) {
+cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t stream,
+                               Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     const bool first = chain_take_first();
     const bool early_start = tuning(EZB_TUNE_PDL) && (!first || tuning(EZB_TUNE_PDL_ACROSS_CALLS));
     attr[0].val.programmaticStreamSerializationAllowed = early_start ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     count_launch();
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    return launch_pdl_cluster(kernel, grid, block, 1, smem, stream, args...);
 }
 }  // namespace ezb

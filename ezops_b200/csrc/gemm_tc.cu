@@ -2,34 +2,28 @@
 //   Y[b, n] = epi( sum_k X[b, k] * W[n, k] ),   2 <= b <= 64,
 // used once the batch turns the weight-streaming GEMV into a skinny GEMM.
 //
-// The weights are still read from HBM exactly once, so the kernel is built like
-// the GEMV -- persistent CTAs, a deep TMA ring, programmatic dependent launch --
-// but the arithmetic moves to tcgen05:
-//   * "swap AB": a tile is 128 weight rows (the MMA's M) by the whole batch
-//     (the MMA's N = 16, 32 or 64) and walks K in blocks of 64 elements;
-//   * one elected thread issues cp.async.bulk.tensor (2-D tiled TMA, 128-byte
-//     swizzle) for the W block [128 x 64] and the X block [N x 64] of a stage;
-//     one elected thread issues tcgen05.mma (kind::f16, bf16 x bf16 -> fp32)
-//     with the accumulator in tensor memory, and tcgen05.commit hands the stage
-//     back to the producer when the MMAs that read it have retired;
-//   * four epilogue warps read the accumulator with tcgen05.ld (thread = weight
-//     row, registers = batch columns) and apply the same epilogues as the GEMV;
-//     the accumulator is double buffered in tensor memory, so the epilogue of
-//     one tile overlaps the MMAs of the next;
-//   * work is split "stream-K": the (tile, k-block) units are dealt evenly to
-//     the CTAs in order, whatever the matrix shape (a 4096-row matrix has only
-//     32 tiles for 148 SMs).  A CTA that covers only part of a tile's K range
-//     stores its fp32 partial tile in the workspace; the last contributor of the
-//     tile (one atomic ticket, no waiting) adds the partials in CTA order, so
-//     results are bit-reproducible.  A CTA works through its shared tiles first
-//     and its whole tiles after them, so that fix-up overlaps their streaming.
-//   * the LINK instance pushes its fp32 results into the tensor-parallel peers'
-//     inboxes instead of storing them (see TpLink).
-// Every mbarrier wait is bounded; on a time-out the CTA records a fault, stops
-// issuing work, waits (bounded) for copies in flight, frees its tensor memory
-// and returns.
+// The weights are read from HBM exactly once and that is what bounds the kernel, so it is built like the GEMV (TMA
+// ring, programmatic dependent launch) with the arithmetic on tcgen05:
+//   * "swap AB": a tile is up to 128 weight rows (the MMA's M) by the whole batch (the MMA's N = 16, 32 or 64) and
+//     walks K in blocks of 64 elements;
+//   * one elected thread issues cp.async.bulk.tensor (2-D tiled TMA, 128-byte swizzle) for the W block [rows x 64]
+//     and the X block [N x 64] of a stage; one elected thread issues tcgen05.mma (kind::f16, bf16 x bf16 -> fp32)
+//     with the accumulator in tensor memory, and tcgen05.commit hands the stage back to the producer when the MMAs
+//     that read it have retired; the accumulator is double buffered, so a tile's epilogue overlaps the next tile;
+//   * K is split over the CTAs of a thread-block cluster (1, 2, 4 or 8).  A CTA writes the batch columns of its
+//     partial tile that belong to CTA j straight from tensor memory into CTA j's shared memory (DSMEM), one mbarrier
+//     arrival per warp and destination; CTA j adds the parts in cluster rank order (fixed order: results are
+//     bit-reproducible) and applies the epilogue to its columns;
+//   * the number of rows of a tile is free (the TMA box is encoded with it), so that the host can deal N rows evenly
+//     to the clusters that fit on the chip (tc_plan below);
+//   * a CTA takes at most half of an SM (shared memory, registers, tensor memory), so that the next kernel of a chain
+//     can be resident while this one drains and already has its weight ring in flight when its input is complete.
+//   * the LINK instance pushes its fp32 results into the tensor-parallel peers' inboxes (see TpLink).
+// Every mbarrier wait is bounded; on a time-out the CTA records a fault, stops issuing work, waits (bounded) for
+// copies in flight, frees its tensor memory and returns.
 #include <cuda.h>
 
+#include <atomic>
 #include <cstring>
 #include <mutex>
 
@@ -37,30 +31,29 @@
 
 namespace ezb {
 
-static constexpr int kTcRows = 128;     // weight rows per tile (MMA M)
+static constexpr int kTcRows = 128;     // MMA M; a tile holds at most this many weight rows
 static constexpr int kTcBlockK = 64;    // k elements per stage: 128 bytes, one swizzle row
-static constexpr int kTcThreads = 192;  // TMA warp, MMA warp, four epilogue warps
-static constexpr int kTcMaxStages = 10;
-static constexpr int kTcMaxSegs = 32;  // tile segments per CTA: at most tiles / CTAs + 2
-static constexpr int kTcABytes = kTcRows * kTcBlockK * 2;
-// Projections of different shapes share one workspace, so the region of the
-// ticket counters (which must stay zero between launches) has one fixed size
-// and never overlaps the partial tiles of another projection.
-static constexpr size_t kTcCounterBytes = 16384;
-static constexpr int kTcMaxTiles = (int)(kTcCounterBytes / 4);
+static constexpr int kTcEpiWarps = 8;
+static constexpr int kTcThreads = 64 + 32 * kTcEpiWarps;  // TMA warp, MMA warp, epilogue warps
+static constexpr int kTcMaxStages = 40;
+static constexpr int kTcMaxCluster = 8;
+static constexpr int kTcTailBytes = 1024;  // barriers, tensor-memory slot, abort flag
 
 struct TcParams {
     int N, K, B;          // output units (rows, or gate/up pairs), reduction length, batch
-    int tiles, kblocks;   // ceil(N / units per tile), ceil(K / 64)
+    int tiles, kblocks;   // ceil(N / units), ceil(K / 64)
+    int units;            // output units per tile (<= 128, or <= 64 pairs)
+    int half_rows;        // pair: first row of the up block inside a tile (units rounded up to 8); else 0
+    int a_rows;           // rows of the W block in a stage, a multiple of 8
+    int log2c;            // log2 of the cluster size
+    int cpc;              // batch columns that one CTA of the cluster finishes
     int nstages;
-    int pair;             // 1: tile = 64 gate rows + 64 up rows, SwiGLU epilogue
+    int pair;             // 1: a tile holds `units` gate rows and `units` up rows, SwiGLU epilogue
     int epilogue;
     const bf16* residual;
     long long ldres;
     void* out;
     long long ldout;
-    float* partial;          // [grid][2][NB][128] fp32 partial tiles
-    unsigned int* counters;  // [tiles], zero between launches
     unsigned int* status;
     Trace trace;
     int trace_id;
@@ -127,49 +120,113 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-// First unit of CTA c when T units are dealt to G CTAs in order.
-__device__ __forceinline__ long long tc_first_unit(long long T, int G, int c) { return T * c / G; }
-// CTA that owns unit u.
-__device__ __forceinline__ int tc_owner(long long T, int G, long long u) {
-    int c = (int)(u * G / T);
-    while (c + 1 < G && tc_first_unit(T, G, c + 1) <= u) ++c;
-    while (c > 0 && tc_first_unit(T, G, c) > u) --c;
-    return c;
+// ---- cluster wrappers -------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// Address of `local` (a shared::cta address) in the shared memory of cluster CTA `rank`.
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Bulk copy from this CTA's shared memory into another CTA's of the cluster; the bytes are counted on that CTA's barrier.
+__device__ __forceinline__ void bulk_s2cluster(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src),
+                 "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// As mbar_wait_bounded, for arrivals from other CTAs of the cluster.
+__device__ __forceinline__ bool mbar_wait_bounded_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                                          unsigned int* status, unsigned int fault_code) {
+    const long long t0 = clock64();
+    while (!mbar_try_wait_cluster(bar, parity)) {
+        if (*abort_flag) return false;
+        if (clock64() - t0 > kWaitLimitCycles) {
+            *abort_flag = 1;
+            report_fault(status, fault_code);
+            return false;
+        }
+    }
+    return true;
 }
 
+// One thread of a converged warp.  Unlike `lane == 0`, the compiler knows that exactly one thread enters the branch and
+// keeps descriptors and addresses in uniform registers: four MMAs and their commit issue in 171 cycles instead of 264.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+
+// 32 lanes x 8 columns, see tmem_ld16
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// What bounds it: the weight stream.  A tile's parts meet in shared memory because the round trips of a reduction
+// through L2 (park, ticket, read 4..19 parts in one CTA) cost 5..13 us at the end of every projection.
+// Measured: Qwen3-8B layer, batch 32, KV 4096 187.9 -> 168.0 us; eight 2B layers, batch 13, paged 680 -> 488 us.
 // LINK: the instance whose epilogue pushes its fp32 results into the peers' inboxes (see TpLink).
 template <int NB, bool LINK>
-__global__ void __launch_bounds__(kTcThreads, 1)
+__global__ void __launch_bounds__(kTcThreads, 2)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant__ CUtensorMap mapW1,
                const __grid_constant__ CUtensorMap mapX, const TcParams p) {
     constexpr int B_BYTES = NB * kTcBlockK * 2;
-    constexpr int STAGE_BYTES = kTcABytes + B_BYTES;
     constexpr int TMEM_COLS = (2 * NB < 32) ? 32 : 2 * NB;  // two accumulators, power of two >= 32
     constexpr uint32_t IDESC = umma_idesc_bf16(kTcRows, NB);
 
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     unsigned char* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);  // swizzled tiles need 1024-byte alignment
+    const uint32_t a_bytes = (uint32_t)p.a_rows * (kTcBlockK * 2);
+    const uint32_t stage_bytes = a_bytes + B_BYTES;
     unsigned char* stages = smem;
-    unsigned char* tail = smem + (size_t)p.nstages * STAGE_BYTES;
+    unsigned char* tail = smem + (size_t)p.nstages * stage_bytes;
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(tail);
     uint64_t* empty_bar = full_bar + kTcMaxStages;
     uint64_t* acc_full = empty_bar + kTcMaxStages;  // [2] accumulator ready for the epilogue
     uint64_t* acc_empty = acc_full + 2;             // [2] accumulator drained
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* recv_full = acc_empty + 2;            // the parts of all CTAs of the cluster have arrived in recv
+    uint64_t* recv_free = recv_full + 1;            // all CTAs of the cluster have read what this CTA sent them
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(recv_free + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    int* ticket = reinterpret_cast<int*>(tmem_slot + 2);
-    float* xch = reinterpret_cast<float*>(tail + 256);  // [64][NB + 1]: up values handed to the gate warps
-    // Segment table of this CTA, in processing order: {tile, first k-block, end k-block, partial slot}.
-    int* segs = reinterpret_cast<int*>(tail + 256 + 64 * (NB + 1) * sizeof(float));
-    int* nseg_s = segs + 4 * kTcMaxSegs;
+    const int RS = p.a_rows;                                                    // rows of a column of a partial tile
+    float* mine = reinterpret_cast<float*>(tail + kTcTailBytes);                // [column][RS]: this CTA's part of the tile
+    float* recv = mine + (size_t)(p.cpc << p.log2c) * RS;                       // [sender][column of this CTA][RS]
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int NS = p.nstages;
-    const int G = gridDim.x, cta = blockIdx.x;
-    const long long T = (long long)p.tiles * p.kblocks;
-    const long long u0 = tc_first_unit(T, G, cta), u1 = tc_first_unit(T, G, cta + 1);
-    const int KB = p.kblocks;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int NS = p.nstages, KB = p.kblocks;
+    const int C = 1 << p.log2c;
+    const int rank = (int)cluster_rank();
+    const int cluster = blockIdx.x >> p.log2c, n_clusters = gridDim.x >> p.log2c;
+    const int kb0 = (int)((long long)KB * rank >> p.log2c), kb1 = (int)((long long)KB * (rank + 1) >> p.log2c);
+    const int my_tiles = (p.tiles - cluster + n_clusters - 1) / n_clusters;
 
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
@@ -178,32 +235,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant_
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(smem_u32(&acc_full[a]), 1);
-            mbar_init(smem_u32(&acc_empty[a]), 4);
+            mbar_init(smem_u32(&acc_empty[a]), kTcEpiWarps);
         }
+        mbar_init(smem_u32(recv_full), 1);
+        mbar_init(smem_u32(recv_free), kTcEpiWarps * C);
         *abort_flag = 0;
         mbar_fence_init();
-        // The unit range [u0, u1) cut at tile boundaries.  Partial tiles (shared with a neighbour CTA) are
-        // processed FIRST, whole tiles after them: the fix-up of a shared tile then runs in the epilogue
-        // warps while the producer and the MMA warp are already streaming the whole tiles, instead of
-        // at the very end of the kernel where nothing can hide it.
-        int n = 0;
-        for (int pass = 0; pass < 2; ++pass) {
-            long long u = u0;
-            int natural = 0;
-            while (u < u1) {
-                const int t = (int)(u / KB), k0 = (int)(u % KB);
-                const long long left = u1 - u;
-                const int k1 = (KB - k0 < left) ? KB : k0 + (int)left;
-                const bool whole = (k0 == 0 && k1 == KB);
-                if ((pass == 0) != whole) {
-                    segs[4 * n] = t, segs[4 * n + 1] = k0, segs[4 * n + 2] = k1, segs[4 * n + 3] = natural == 0 ? 0 : 1;
-                    ++n;
-                }
-                u += k1 - k0;
-                ++natural;
-            }
-        }
-        *nseg_s = n;
     }
     if (warp == 1) {
         tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
@@ -215,58 +252,48 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant_
     const uint32_t tmem_base = *tmem_slot;
     unsigned long long* trec = (tid == 64) ? trace_open(p.trace, (unsigned)p.trace_id, blockIdx.x) : nullptr;
     pdl_trigger();
+    // The barriers above are initialised: peers may write here once they have passed the wait.  (A launch without a
+    // cluster leaves the cluster barrier alone: there its wait held the epilogue until every warp of the CTA had come.)
+    if (C > 1) cluster_arrive();
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            // One thread feeds the whole ring, so its per-unit cost matters: all counters
-            // are 32-bit and advance incrementally (no divisions in the loop).
-            const int n_units = (int)(u1 - u0);
-            const int nseg = *nseg_s;
-            // two cursors over the segment table: the next unit whose weights / activations are requested
-            int wsi = 0, wkb = nseg ? segs[1] : 0, xsi = 0, xkb = wkb;
-            auto advance = [&](int& si, int& kb) {
-                if (++kb == segs[4 * si + 2]) {
-                    ++si;
-                    kb = si < nseg ? segs[4 * si + 1] : 0;
-                }
-            };
+        if (elect_one()) {
+            const int n_units = my_tiles * (kb1 - kb0);
+            const int box_rows = p.pair ? 2 * p.units : p.units;
+            const uint32_t tx = (uint32_t)box_rows * (kTcBlockK * 2) + B_BYTES;
+            // Two cursors over (tile, k-block): the next unit whose weights / activations are requested.  The clusters
+            // start their walk along K at different blocks: in step, all of them would ask the same few lines of X of
+            // the L2 at the same time (a k-block took 270 ns however small its tile).
+            const int k_first = kb0 + (int)((long long)(kb1 - kb0) * cluster / n_clusters);
+            int wt = cluster, wkb = k_first, xkb = k_first;
             int stage = 0;
             uint32_t empty_parity = 1;  // a fresh barrier passes a wait on parity 1
-            auto request_w = [&](int st, int t, int k) {
+            auto request_w = [&](int st) {
                 const uint32_t bar = smem_u32(&full_bar[st]);
-                mbar_arrive_expect_tx(bar, STAGE_BYTES);
-                const uint32_t a = smem_u32(stages + (size_t)st * STAGE_BYTES);
-                if (p.pair) {
-                    tma_load_2d(a, &mapW0, k * kTcBlockK, t * (kTcRows / 2), bar);
-                    tma_load_2d(a + kTcABytes / 2, &mapW1, k * kTcBlockK, t * (kTcRows / 2), bar);
-                } else {
-                    tma_load_2d(a, &mapW0, k * kTcBlockK, t * kTcRows, bar);
-                }
+                mbar_arrive_expect_tx(bar, tx);
+                const uint32_t a = smem_u32(stages) + (uint32_t)st * stage_bytes;
+                tma_load_2d(a, &mapW0, wkb * kTcBlockK, wt * p.units, bar);
+                if (p.pair) tma_load_2d(a + (uint32_t)p.half_rows * (kTcBlockK * 2), &mapW1, wkb * kTcBlockK, wt * p.units, bar);
+                if (++wkb == kb1) wkb = kb0;
+                if (wkb == k_first) wt += n_clusters;
             };
-            auto request_x = [&](int st, int k) {
-                tma_load_2d(smem_u32(stages + (size_t)st * STAGE_BYTES) + kTcABytes, &mapX, k * kTcBlockK, 0,
-                            smem_u32(&full_bar[st]));
+            auto request_x = [&](int st) {
+                tma_load_2d(smem_u32(stages) + (uint32_t)st * stage_bytes + a_bytes, &mapX, xkb * kTcBlockK, 0, smem_u32(&full_bar[st]));
+                if (++xkb == kb1) xkb = kb0;
             };
             // weights do not depend on the kernel in front: request them before the dependency wait
             const int npre = n_units < NS ? n_units : NS;
-            for (int i = 0; i < npre; ++i) {
-                request_w(i, segs[4 * wsi], wkb);
-                advance(wsi, wkb);
-            }
+            for (int i = 0; i < npre; ++i) request_w(i);
             pdl_wait();
-            for (int i = 0; i < npre; ++i) {
-                request_x(i, xkb);
-                advance(xsi, xkb);
-            }
+            for (int i = 0; i < npre; ++i) request_x(i);
             int issued = npre;
             stage = (npre == NS) ? 0 : npre;
             if (npre == NS) empty_parity = 0;
             for (int i = npre; i < n_units; ++i) {
                 if (!mbar_wait_bounded(smem_u32(&empty_bar[stage]), empty_parity, abort_flag, p.status, FAULT_GEMV_EMPTY_WAIT)) break;
-                request_w(stage, segs[4 * wsi], wkb);
-                request_x(stage, wkb);
-                advance(wsi, wkb);
+                request_w(stage);
+                request_x(stage);
                 if (++stage == NS) stage = 0, empty_parity ^= 1;
                 issued = i + 1;
             }
@@ -284,16 +311,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant_
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            const int nseg = *nseg_s;
+        if (elect_one()) {
             int stage = 0;
             uint32_t full_parity = 0;
-            for (int seg = 0; seg < nseg && !(*abort_flag); ++seg) {
-                const int kb0 = segs[4 * seg + 1], kb1 = segs[4 * seg + 2];
-                const int acc = seg & 1;
+            for (int i = 0; i < my_tiles && !(*abort_flag); ++i) {
+                const int acc = i & 1;
                 // wait until the epilogue has drained this accumulator (passes at once for its first use)
-                if (!mbar_wait_bounded(smem_u32(&acc_empty[acc]), (uint32_t)(((seg >> 1) & 1) ^ 1), abort_flag, p.status,
-                                       FAULT_TC_ACC_WAIT))
+                if (!mbar_wait_bounded(smem_u32(&acc_empty[acc]), (uint32_t)(((i >> 1) & 1) ^ 1), abort_flag, p.status, FAULT_TC_ACC_WAIT))
                     break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(acc * NB);
@@ -301,9 +325,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant_
                     if (!mbar_wait_bounded(smem_u32(&full_bar[stage]), full_parity, abort_flag, p.status, FAULT_GEMV_FULL_WAIT))
                         break;
                     tc_fence_after();
-                    const uint32_t a_addr = smem_u32(stages + (size_t)stage * STAGE_BYTES);
+                    const uint32_t a_addr = smem_u32(stages) + (uint32_t)stage * stage_bytes;
                     const uint64_t adesc = umma_desc_sw128(a_addr);
-                    const uint64_t bdesc = umma_desc_sw128(a_addr + kTcABytes);
+                    const uint64_t bdesc = umma_desc_sw128(a_addr + a_bytes);
+                    // A tile with fewer than 128 rows is multiplied as if it had 128: the rows behind it are whatever
+                    // the shared memory holds, and the accumulator lanes they end up in are never read.
 #pragma unroll
                     for (int k = 0; k < kTcBlockK / 16; ++k)  // 32 bytes along K per MMA: +2 in the 16-byte address field
                         tc_mma_bf16(d_tmem, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
@@ -315,198 +341,148 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant_
         }
     } else {
         // ------------------------------------------------------------ epilogue warps
-        const int q = warp & 3;          // tensor-memory lane quarter this warp may read
-        const int row = q * 32 + lane;   // row of the tile held by this thread
+        const int q = warp & 3;            // tensor-memory lane quarter this warp may read
+        const int row = q * 32 + lane;     // row of the tile held by this thread
         const int et = (warp - 2) * 32 + lane;
+        constexpr int HC = NB / 2;         // two warps share a lane quarter: each drains half of the batch columns
+        const int b_half = ((warp - 2) >> 2) * HC;
+        const int cpc = p.cpc;  // batch columns per CTA of the cluster
+        auto cols_of = [&](int r) { return max(0, min(cpc, p.B - r * cpc)); };
+        const int b_first = rank * cpc, n_cols = cols_of(rank);
+        // the threads that finish a tile: a row (or pair) each, every `groups`-th column
+        const int frow = p.pair ? (et & 63) : (et & 127);
+        const int cg = p.pair ? (et >> 6) : (et >> 7), groups = p.pair ? 4 : 2;
+        if (C > 1) cluster_wait();
         pdl_wait();
         trace_mark(trec, 3);
         const unsigned int push_epoch = (LINK && p.link.world > 0 && p.link.push_inbox >= 0) ? tp_next_epoch(p.link, p.link.push_inbox) : 0u;
         const bool poisoned = LINK && p.link.world > 0 && tp_poisoned(p.status);  // see tp_poisoned: push nothing, advance nothing
-        const int nseg = *nseg_s;
-        for (int seg = 0; seg < nseg; ++seg) {
-            const int tile = segs[4 * seg], kb0 = segs[4 * seg + 1], kb1 = segs[4 * seg + 2];
-            const int acc = seg & 1;
-            mbar_wait_bounded(smem_u32(&acc_full[acc]), (uint32_t)((seg >> 1) & 1), abort_flag, p.status, FAULT_TC_ACC_WAIT);
-            if (seg == 0) trace_mark(trec, 4);
+        for (int i = 0; i < my_tiles; ++i) {
+            const int tile = cluster + i * n_clusters;
+            const int acc = i & 1;
+            const int n = tile * p.units + frow;
+            const bool live_row = frow < p.units && n < p.N;
+            constexpr int CU = 4;  // columns in flight per thread
+            // residual values of the first columns are fetched while the tile is still being multiplied
+            float res[CU];
+            auto fetch_residual = [&](int col) {
+                const bf16* src = p.residual + (long long)(b_first + col) * p.ldres + n;
+#pragma unroll
+                for (int u = 0; u < CU; ++u) {
+                    if (col + u * groups < n_cols) res[u] = __bfloat162float(*src);
+                    src += groups * p.ldres;
+                }
+            };
+            if (p.epilogue == EPI_RESIDUAL && live_row) fetch_residual(cg);
+            mbar_wait_bounded(smem_u32(&acc_full[acc]), (uint32_t)((i >> 1) & 1), abort_flag, p.status, FAULT_TC_ACC_WAIT);
+            if (i == 0) trace_mark(trec, 4);
             tc_fence_after();
-            float v[NB];
+            if (i > 0)  // the previous tile's parts have been read, here and by the CTAs they were sent to
+                mbar_wait_bounded_cluster(smem_u32(recv_free), (uint32_t)((i - 1) & 1), abort_flag, p.status, FAULT_TC_ACC_WAIT);
+            const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * NB + b_half);
+            float* dst = mine + (size_t)b_half * RS + row;
+            const int b_left = p.B - b_half;
+            if constexpr (HC == 8) {
+                float v[8];
+                tmem_ld8(t_addr, v);
+                tmem_ld_wait();
+                if (row < RS) {
 #pragma unroll
-            for (int c = 0; c < NB; c += 16) {
-                float t[16];
-                tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * NB + c), t);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[c + i] = t[i];
-            }
-            tmem_ld_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&acc_empty[acc]));
-
-            const bool whole = (kb0 == 0 && kb1 == KB);
-            if (!whole) {
-                bool finish;
-                // partial tile: park it, take a ticket; the last contributor adds all parts in CTA order
-                float* mine = p.partial + ((size_t)cta * 2 + segs[4 * seg + 3]) * (NB * kTcRows);
-#pragma unroll
-                for (int b = 0; b < NB; ++b) mine[b * kTcRows + row] = v[b];
-                named_bar_sync(2, 128);
-                const long long t_first = (long long)tile * KB, t_last = t_first + KB - 1;
-                const int c_first = tc_owner(T, G, t_first), c_last = tc_owner(T, G, t_last);
-                if (et == 0) {
-                    unsigned int prev;
-                    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(p.counters + tile) : "memory");
-                    *ticket = (prev == (unsigned int)(c_last - c_first)) ? 1 : 0;
-                    if (*ticket) p.counters[tile] = 0u;
-                }
-                named_bar_sync(2, 128);
-                finish = (*ticket != 0);
-                named_bar_sync(2, 128);  // `ticket` may be rewritten by the next segment
-                if (!finish || *abort_flag) continue;
-
-                // Fix-up by the last contributor.  Every value now comes from the parked parts, so the
-                // threads regroup for memory-level parallelism: a thread owns 4 consecutive rows
-                // (one 16-byte load per part and batch row) of a quarter of the batch, and the parts
-                // of two contributors are in flight together.  Parts are added in CTA order, which
-                // fixes the bits whatever the arrival order was.
-                constexpr int NBG = NB / 4;
-                const int r4 = lane * 4, b0 = (et >> 5) * NBG;
-                float4 acc[NBG];
-#pragma unroll
-                for (int j = 0; j < NBG; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 2
-                for (int c = c_first; c <= c_last; ++c) {
-                    const bool first_seg = (tc_first_unit(T, G, c) / KB) == tile;
-                    const float* part = p.partial + ((size_t)c * 2 + (first_seg ? 0 : 1)) * (NB * kTcRows) + b0 * kTcRows + r4;
-#pragma unroll
-                    for (int j = 0; j < NBG; ++j) {
-                        const float4 t = __ldcg(reinterpret_cast<const float4*>(part + j * kTcRows));
-                        acc[j].x += t.x, acc[j].y += t.y, acc[j].z += t.z, acc[j].w += t.w;
-                    }
-                }
-                if (LINK && !p.pair && p.epilogue == EPI_PUSH_F32) {
-                    // A lane holds 4 consecutive rows; stored as they are, a warp's 64-bit peer stores would
-                    // be 32 bytes apart (one NVLink transaction each: measured 30 us per tile).  Shuffle so
-                    // that lane L owns rows 2L, 2L+1 (then 64+2L, 64+2L+1): 512 contiguous bytes per store.
-                    const int src = lane >> 1;
-                    const bool odd = lane & 1;
-#pragma unroll
-                    for (int j = 0; j < NBG; ++j) {
-#pragma unroll
-                        for (int half = 0; half < 2; ++half) {
-                            const int s2 = src + half * 16;
-                            const float ax = __shfl_sync(0xffffffffu, acc[j].x, s2), ay = __shfl_sync(0xffffffffu, acc[j].y, s2);
-                            const float az = __shfl_sync(0xffffffffu, acc[j].z, s2), aw = __shfl_sync(0xffffffffu, acc[j].w, s2);
-                            if (!poisoned && b0 + j < p.B && tile * kTcRows + half * 64 + 2 * lane < p.N)
-                                tp_push2(p.link, (long long)(b0 + j) * p.ldout + tile * kTcRows + half * 64 + 2 * lane,
-                                         odd ? az : ax, odd ? aw : ay, push_epoch);
-                        }
-                    }
-                    continue;
-                }
-                if (!p.pair) {
-                    const int n = tile * kTcRows + r4;
-                    if (n < p.N) {
-                        if (p.epilogue == EPI_RESIDUAL) {
-                            uint2 res[NBG];
-#pragma unroll
-                            for (int j = 0; j < NBG; ++j)
-                                res[j] = (b0 + j < p.B) ? *reinterpret_cast<const uint2*>(p.residual + (long long)(b0 + j) * p.ldres + n)
-                                                        : make_uint2(0u, 0u);
-#pragma unroll
-                            for (int j = 0; j < NBG; ++j)
-                                if (b0 + j < p.B)
-                                    *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(p.out) + (long long)(b0 + j) * p.ldout + n) =
-                                        make_uint2(pack_bf16(bf16_lo(res[j].x) + round_bf16(acc[j].x), bf16_hi(res[j].x) + round_bf16(acc[j].y)),
-                                                   pack_bf16(bf16_lo(res[j].y) + round_bf16(acc[j].z), bf16_hi(res[j].y) + round_bf16(acc[j].w)));
-                        } else if (p.epilogue == EPI_STORE_F32) {
-#pragma unroll
-                            for (int j = 0; j < NBG; ++j)
-                                if (b0 + j < p.B) *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + (long long)(b0 + j) * p.ldout + n) = acc[j];
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < NBG; ++j)
-                                if (b0 + j < p.B)
-                                    *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(p.out) + (long long)(b0 + j) * p.ldout + n) =
-                                        make_uint2(pack_bf16(acc[j].x, acc[j].y), pack_bf16(acc[j].z, acc[j].w));
-                        }
-                    }
-                } else {
-                    // lanes 0..15 hold gate rows 0..63, lanes 16..31 the matching up rows
-                    const int n = tile * (kTcRows / 2) + r4;
-#pragma unroll
-                    for (int j = 0; j < NBG; ++j) {
-                        float4 up;
-                        up.x = __shfl_down_sync(0xffffffffu, acc[j].x, 16), up.y = __shfl_down_sync(0xffffffffu, acc[j].y, 16);
-                        up.z = __shfl_down_sync(0xffffffffu, acc[j].z, 16), up.w = __shfl_down_sync(0xffffffffu, acc[j].w, 16);
-                        if (lane < 16 && n < p.N && b0 + j < p.B) {
-                            const float o0 = round_bf16(silu_f32(round_bf16(acc[j].x))) * round_bf16(up.x);
-                            const float o1 = round_bf16(silu_f32(round_bf16(acc[j].y))) * round_bf16(up.y);
-                            const float o2 = round_bf16(silu_f32(round_bf16(acc[j].z))) * round_bf16(up.z);
-                            const float o3 = round_bf16(silu_f32(round_bf16(acc[j].w))) * round_bf16(up.w);
-                            *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(p.out) + (long long)(b0 + j) * p.ldout + n) =
-                                make_uint2(pack_bf16(o0, o1), pack_bf16(o2, o3));
-                        }
-                    }
-                }
-                continue;
-            }
-            if (*abort_flag) continue;
-
-            if (!p.pair) {
-                const int n = tile * kTcRows + row;
-                if (n < p.N) {
-                    if (p.epilogue == EPI_RESIDUAL) {
-                        // all residual values are fetched before the first store: the stores may alias
-                        // them as far as the compiler knows, which would serialise 64 L2 round trips
-                        float res[NB];
-#pragma unroll
-                        for (int b = 0; b < NB; ++b)
-                            res[b] = (b < p.B) ? __bfloat162float(p.residual[(long long)b * p.ldres + n]) : 0.f;
-#pragma unroll
-                        for (int b = 0; b < NB; ++b)
-                            if (b < p.B)
-                                reinterpret_cast<bf16*>(p.out)[(long long)b * p.ldout + n] =
-                                    __float2bfloat16_rn(res[b] + round_bf16(v[b]));
-                    } else if (LINK && p.epilogue == EPI_PUSH_F32) {
-#pragma unroll
-                        for (int b = 0; b < NB; ++b)
-                            if (b < p.B && !poisoned) tp_push(p.link, (long long)b * p.ldout + n, v[b], push_epoch);
-                    } else if (p.epilogue == EPI_STORE_F32) {
-#pragma unroll
-                        for (int b = 0; b < NB; ++b)
-                            if (b < p.B) reinterpret_cast<float*>(p.out)[(long long)b * p.ldout + n] = v[b];
-                    } else {
-#pragma unroll
-                        for (int b = 0; b < NB; ++b)
-                            if (b < p.B) reinterpret_cast<bf16*>(p.out)[(long long)b * p.ldout + n] = __float2bfloat16_rn(v[b]);
-                    }
+                    for (int e = 0; e < 8; ++e, dst += RS)
+                        if (e < b_left) *dst = v[e];
                 }
             } else {
-                // rows 0..63 hold gate values of pairs 0..63, rows 64..127 the matching up values
-                if (row >= 64) {
 #pragma unroll
-                    for (int b = 0; b < NB; ++b) xch[(row - 64) * (NB + 1) + b] = v[b];
-                }
-                named_bar_sync(2, 128);
-                if (row < 64) {
-                    const int n = tile * (kTcRows / 2) + row;
-                    if (n < p.N) {
+                for (int c = 0; c < HC; c += 16) {
+                    float v[16];
+                    tmem_ld16(t_addr + (uint32_t)c, v);
+                    tmem_ld_wait();
+                    if (row < RS) {
 #pragma unroll
-                        for (int b = 0; b < NB; ++b) {
-                            if (b >= p.B) break;
-                            const float gate = round_bf16(v[b]), up = round_bf16(xch[row * (NB + 1) + b]);
-                            reinterpret_cast<bf16*>(p.out)[(long long)b * p.ldout + n] =
-                                __float2bfloat16_rn(round_bf16(silu_f32(gate)) * up);
-                        }
+                        for (int e = 0; e < 16; ++e, dst += RS)
+                            if (c + e < b_left) *dst = v[e];
                     }
                 }
-                named_bar_sync(2, 128);
+            }
+            tc_fence_before();
+            fence_async_shared();
+            named_bar_sync(2, 32 * kTcEpiWarps);
+            if (lane == 0) mbar_arrive(smem_u32(&acc_empty[acc]));
+            if (C > 1) {
+                if (warp == 2) {  // one lane per destination
+                    if (lane == 0) mbar_arrive_expect_tx(smem_u32(recv_full), (uint32_t)((C - 1) * n_cols * RS * 4));
+                    const uint32_t bytes = lane < C ? (uint32_t)(cols_of(lane) * RS * 4) : 0u;
+                    if (lane != rank && bytes && !*abort_flag)
+                        bulk_s2cluster(map_to_rank(smem_u32(recv + (size_t)rank * cpc * RS), lane), smem_u32(mine + (size_t)lane * cpc * RS), bytes,
+                                       map_to_rank(smem_u32(recv_full), lane));
+                    __syncwarp();
+                }
+                mbar_wait_bounded(smem_u32(recv_full), (uint32_t)(i & 1), abort_flag, p.status, FAULT_TC_ACC_WAIT);
+            }
+            // The parts of columns col, col + groups, ... of this thread's row, added in rank order
+            auto gather = [&](int col, int first_row, float (&v)[CU]) {
+#pragma unroll
+                for (int u = 0; u < CU; ++u) v[u] = 0.f;
+                for (int s = 0; s < C; ++s) {
+                    const float* part = (s == rank ? mine : recv) + (size_t)(s * cpc + col) * RS + first_row;
+#pragma unroll
+                    for (int u = 0; u < CU; ++u)
+                        if (col + u * groups < n_cols) v[u] += part[u * groups * RS];
+                }
+            };
+            if (!*abort_flag && live_row) {
+                float v[CU];
+                const long long step = (long long)groups * p.ldout;
+                for (int col = cg; col < n_cols; col += CU * groups) {
+                    const long long o = (long long)(b_first + col) * p.ldout + n;
+                    gather(col, frow, v);
+                    if (p.pair) {
+                        float up[CU];
+                        gather(col, frow + p.half_rows, up);
+                        bf16* out = reinterpret_cast<bf16*>(p.out) + o;
+#pragma unroll
+                        for (int u = 0; u < CU; ++u, out += step)
+                            if (col + u * groups < n_cols) *out = __float2bfloat16_rn(round_bf16(silu_f32(round_bf16(v[u]))) * round_bf16(up[u]));
+                    } else if (p.epilogue == EPI_RESIDUAL) {
+                        if (col != cg) fetch_residual(col);
+                        bf16* out = reinterpret_cast<bf16*>(p.out) + o;
+#pragma unroll
+                        for (int u = 0; u < CU; ++u, out += step)
+                            if (col + u * groups < n_cols) *out = __float2bfloat16_rn(res[u] + round_bf16(v[u]));
+                    } else if (LINK && p.epilogue == EPI_PUSH_F32) {
+#pragma unroll
+                        for (int u = 0; u < CU; ++u)
+                            if (!poisoned && col + u * groups < n_cols) tp_push(p.link, o + u * step, v[u], push_epoch);
+                    } else if (p.epilogue == EPI_STORE_F32) {
+                        float* out = reinterpret_cast<float*>(p.out) + o;
+#pragma unroll
+                        for (int u = 0; u < CU; ++u, out += step)
+                            if (col + u * groups < n_cols) *out = v[u];
+                    } else {
+                        bf16* out = reinterpret_cast<bf16*>(p.out) + o;
+#pragma unroll
+                        for (int u = 0; u < CU; ++u, out += step)
+                            if (col + u * groups < n_cols) *out = __float2bfloat16_rn(v[u]);
+                    }
+                }
+            }
+            if (i + 1 < my_tiles) {
+                __syncwarp();
+                if (lane < C) mbar_arrive_cluster(map_to_rank(smem_u32(recv_free), lane));
             }
         }
         trace_mark(trec, 5);
         if (LINK && p.link.world > 0 && p.link.bump_inbox >= 0 && blockIdx.x == 0 && et == 0 && !*abort_flag && !poisoned) tp_bump(p.link);
     }
 
+    __syncwarp();
+    if (C > 1 && warp < 2) cluster_wait();
+    if (*abort_flag) __nanosleep(200000);  // copies towards the peers that may still be in flight
+    // No CTA of the cluster leaves while another may still write to it or signal it.
+    if (C > 1) {
+        cluster_arrive();
+        cluster_wait();
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
@@ -586,78 +562,139 @@ static bool make_map(CUtensorMap* map, const bf16* base, long long rows, long lo
 static int tc_batch_tile(int B) { return B <= 16 ? 16 : (B <= 32 ? 32 : 64); }
 
 bool gemm_tc_supported(int B, int K) { return B >= 2 && B <= 64 && K % 8 == 0 && encode_fn() != nullptr; }
-bool gemm_tc_fits(int N, bool pair) { return (N + (pair ? 63 : 127)) / (pair ? 64 : 128) <= kTcMaxTiles; }
 
-size_t gemm_tc_workspace_bytes(int B, int N, bool pair) {
-    (void)N, (void)pair;
-    const int NB = tc_batch_tile(B);
-    return kTcCounterBytes + (size_t)sm_count() * 2 * NB * kTcRows * sizeof(float);
+static constexpr size_t kTcHalfSm = 113 * 1024;  // two CTAs of this size share an SM
+
+// Clusters of 1 << log2c CTAs, one CTA per SM, that can be resident together (asked once per device): the clusters of
+// eight leave SMs of a GPC over, 15 of them fit at a whole SM per CTA and 16 at half an SM; 33 of four, 74 of two.
+template <int NB, bool LINK>
+static int tc_resident_clusters(int dev, int log2c, bool half) {
+    static std::atomic<int> cache[64][4][2];
+    const bool keep = dev >= 0 && dev < 64;
+    if (keep)
+        if (const int known = cache[dev][log2c][half].load(std::memory_order_relaxed)) return known;
+    auto ask = [&](size_t smem) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        cfg.gridDim = dim3(1u << log2c);
+        cfg.blockDim = dim3(kTcThreads);
+        cfg.dynamicSmemBytes = smem;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1u << log2c, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        return cudaOccupancyMaxActiveClusters(&n, gemm_tc_kernel<NB, LINK>, &cfg) == cudaSuccess ? n : 0;
+    };
+    int n = ask((size_t)max_smem_optin());
+    if (half) {
+        const int shared = ask(kTcHalfSm) / 2;
+        if (shared > n) n = shared;
+    }
+    const int most = sm_count() >> log2c;
+    if (n > most) n = most;
+    if (n < 1) n = log2c == 0 ? 1 : 0;
+    if (keep && n > 0) cache[dev][log2c][half].store(n, std::memory_order_relaxed);
+    return n;
+}
+
+// How N output units and K are dealt out: cluster size, rows of a tile, rounds of tiles per cluster.  Few rows per CTA
+// waste time per k-block and read X once per tile; large clusters leave SMs idle and exchange more; a second round adds
+// an epilogue where the tile is short.  The estimate below (in ns) weighs these against each other; its constants were
+// fitted to a sweep of every projection over all cluster sizes (Qwen3 0.6B / 2B / 8B / 32B, batch 2..64; e.g. 8B at batch
+// 32, layer us with clusters of 1 | 2 | 4 | 8: gate/up 174.5 | 168.9 | 171.1 | 185.1, down 191.4 | 175.0 | 171.0 | 172.3;
+// 0.6B o_proj 64.9 | 60.5 | 58.6 | 58.4).  A k-block costs 40 ns plus its bytes at a 148th of the HBM rate (never less
+// than 95 ns: the MMAs read 128 rows of A from shared memory whatever the tile holds).
+template <int NB, bool LINK>
+static bool tc_plan(TcParams& p, int dev, int& clusters, size_t& smem) {
+    double best = 0.;
+    for (int log2c = 0; (1 << log2c) <= kTcMaxCluster && (1 << log2c) <= p.kblocks; ++log2c) {
+        const int C = 1 << log2c, max_units = p.pair ? kTcRows / 2 : kTcRows;
+        const int cpc = (p.B + C - 1) / C, nk = (p.kblocks + C - 1) / C;
+        for (int half = 0; half < 2; ++half) {
+            const int nc = tc_resident_clusters<NB, LINK>(dev, log2c, half != 0);
+            if (nc < 1) continue;
+            long long rounds = (p.N + (long long)nc * max_units - 1) / ((long long)nc * max_units);
+            int units = (int)((p.N + nc * rounds - 1) / (nc * rounds));
+            if (units < 8) units = 8;  // a TMA box no smaller than one swizzle group
+            const int half_rows = p.pair ? (units + 7) / 8 * 8 : 0;
+            const int a_rows = p.pair ? 2 * half_rows : (units + 7) / 8 * 8;
+            const int tiles = (int)((p.N + units - 1) / units);
+            const size_t stage = (size_t)(a_rows + NB) * kTcBlockK * 2;
+            const size_t tail = kTcTailBytes + (size_t)(C > 1 ? 2 : 1) * cpc * C * a_rows * sizeof(float);
+            // the MMA reads 128 rows from the start of every stage, whatever a_rows is
+            const size_t a_read = (size_t)kTcRows * kTcBlockK * 2;
+            const size_t behind = stage + tail < a_read ? a_read - stage : tail;
+            const size_t cap = half ? kTcHalfSm : (size_t)max_smem_optin();
+            if (cap < 1024 + behind + 2 * stage) continue;
+            long long ns = (long long)((cap - 1024 - behind) / stage);
+            if (ns > kTcMaxStages) ns = kTcMaxStages;
+            const bool all = ns >= rounds * nk;  // the ring holds everything the CTA reads
+            if (all) ns = rounds * nk < 2 ? 2 : rounds * nk;
+            if (half && !all) continue;  // a long stream wants the deeper ring
+            const double block = 40. + 2.6 * (p.pair ? 2 * units : units) + 0.9 * NB;
+            const double tile = nk * (block < 95. ? 95. : block), epi = (C > 1 ? 1500. : 500.) + 60. * cpc;
+            const double cost = rounds * tile + (rounds - 1) * (epi > tile ? epi - tile : 0.) + epi;
+            if (best > 0. && cost >= best) continue;
+            best = cost;
+            p.log2c = log2c, p.cpc = cpc, p.units = units, p.half_rows = half_rows, p.a_rows = a_rows, p.tiles = tiles;
+            p.nstages = (int)ns;
+            clusters = tiles < nc ? tiles : nc;
+            smem = 1024 + (size_t)ns * stage + behind;
+        }
+    }
+    return best > 0.;
 }
 
 template <int NB, bool LINK>
-static cudaError_t launch_tc_instance(const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap& mx, TcParams& p,
-                                      int grid, cudaStream_t stream) {
+static cudaError_t launch_tc_instance(const GemvArgs& a, const bf16* x, long long ldx, TcParams& p, cudaStream_t stream) {
     auto kernel = gemm_tc_kernel<NB, LINK>;
-    constexpr size_t stage = kTcABytes + (size_t)NB * kTcBlockK * 2;
-    const size_t tail = 256 + (size_t)64 * (NB + 1) * sizeof(float) + (4 * kTcMaxSegs + 4) * sizeof(int);
-    const size_t cap = (size_t)max_smem_optin();
-    int ns = (int)((cap - 1024 - tail) / stage);
-    if (ns > kTcMaxStages) ns = kTcMaxStages;
-    p.nstages = ns;
-    const size_t smem = 1024 + (size_t)ns * stage + tail;
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap);
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin());
         if (e != cudaSuccess) return e;
-        configured[dev] = true;
+        if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    return launch_pdl(kernel, dim3(grid), dim3(kTcThreads), smem, stream, m0, m1, mx, p);
+    int clusters = 0;
+    size_t smem = 0;
+    if (!tc_plan<NB, LINK>(p, dev, clusters, smem)) return cudaErrorInvalidConfiguration;
+    alignas(64) CUtensorMap m0, m1, mx;
+    if (!make_map(&m0, a.W0, a.N, a.K, a.ldw, p.units)) return cudaErrorInvalidValue;
+    if (!make_map(&m1, p.pair ? a.W1 : a.W0, a.N, a.K, a.ldw, p.units)) return cudaErrorInvalidValue;
+    if (!make_map(&mx, x, a.B, a.K, ldx, NB)) return cudaErrorInvalidValue;
+    return launch_pdl_cluster(kernel, dim3((unsigned)clusters << p.log2c), dim3(kTcThreads), 1 << p.log2c, smem, stream, m0, m1, mx, p);
 }
 
 // x must already hold what the MMA consumes (any norm prologue has been run by the caller).
-cudaError_t launch_gemm_tc(const GemvArgs& a, const bf16* x, long long ldx, void* workspace, cudaStream_t stream) {
+cudaError_t launch_gemm_tc(const GemvArgs& a, const bf16* x, long long ldx, cudaStream_t stream) {
     const bool pair = a.epilogue == EPI_SWIGLU;
-    const int NB = tc_batch_tile(a.B);
     TcParams p;
     p.N = a.N, p.K = a.K, p.B = a.B;
-    p.tiles = (a.N + (pair ? 63 : 127)) / (pair ? 64 : 128);
     p.kblocks = (a.K + kTcBlockK - 1) / kTcBlockK;
     p.pair = pair ? 1 : 0;
     p.epilogue = a.epilogue;
     p.residual = a.residual, p.ldres = a.ldres;
     p.out = a.out, p.ldout = a.ldout;
-    if (p.tiles > kTcMaxTiles) return cudaErrorInvalidValue;
-    p.counters = reinterpret_cast<unsigned int*>(workspace);
-    p.partial = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + kTcCounterBytes);
     p.status = status_ptr();
     if (!p.status) return cudaErrorUnknown;
     p.trace = trace_handle();
     p.trace_id = a.trace_id;
     p.link = a.link;
     if (a.link.world > 0 && (a.link.gather_inbox >= 0 || pair)) return cudaErrorNotSupported;  // only the push side lives here
-
-    alignas(64) CUtensorMap m0, m1, mx;
-    const int box_rows = pair ? 64 : 128;
-    if (!make_map(&m0, a.W0, a.N, a.K, a.ldw, box_rows)) return cudaErrorInvalidValue;
-    if (!make_map(&m1, pair ? a.W1 : a.W0, a.N, a.K, a.ldw, box_rows)) return cudaErrorInvalidValue;
-    if (!make_map(&mx, x, a.B, a.K, ldx, NB)) return cudaErrorInvalidValue;
-
-    long long T = (long long)p.tiles * p.kblocks;
-    int grid = sm_count();
-    if (grid > T) grid = (int)T;
+    const int NB = tc_batch_tile(a.B);
     if (a.link.world > 0) {
         switch (NB) {
-            case 16: return launch_tc_instance<16, true>(m0, m1, mx, p, grid, stream);
-            case 32: return launch_tc_instance<32, true>(m0, m1, mx, p, grid, stream);
-            default: return launch_tc_instance<64, true>(m0, m1, mx, p, grid, stream);
+            case 16: return launch_tc_instance<16, true>(a, x, ldx, p, stream);
+            case 32: return launch_tc_instance<32, true>(a, x, ldx, p, stream);
+            default: return launch_tc_instance<64, true>(a, x, ldx, p, stream);
         }
     }
     switch (NB) {
-        case 16: return launch_tc_instance<16, false>(m0, m1, mx, p, grid, stream);
-        case 32: return launch_tc_instance<32, false>(m0, m1, mx, p, grid, stream);
-        default: return launch_tc_instance<64, false>(m0, m1, mx, p, grid, stream);
+        case 16: return launch_tc_instance<16, false>(a, x, ldx, p, stream);
+        case 32: return launch_tc_instance<32, false>(a, x, ldx, p, stream);
+        default: return launch_tc_instance<64, false>(a, x, ldx, p, stream);
     }
 }
 

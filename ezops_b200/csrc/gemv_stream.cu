@@ -912,7 +912,7 @@ cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream) {
     p.trace_id = a.trace_id;
     p.link = a.link;
 
-    const bool use_tc = !rows8 && a.tc_workspace && tuning(EZB_TUNE_TC) != 0 && gemm_tc_supported(a.B, a.K) && gemm_tc_fits(a.N, pair);
+    const bool use_tc = !rows8 && a.allow_tc && tuning(EZB_TUNE_TC) != 0 && gemm_tc_supported(a.B, a.K);
     // The fused tensor-parallel exchange lives in the small-batch kernel (gather and push) and, for larger
     // batches, in the row kernel (gather) and the tensor-core kernel (push); the general fallback has none.
     const bool linked = a.link.world > 0;
@@ -939,7 +939,7 @@ cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream) {
         p.x = a.xn_scratch, p.ldx = a.K;
         p.prologue = PRO_NONE;
     }
-    if (use_tc) return launch_gemm_tc(tc_args, p.x, p.ldx, a.tc_workspace, stream);
+    if (use_tc) return launch_gemm_tc(tc_args, p.x, p.ldx, stream);
 
     if (rows8) {
         const int which = (pair ? 4 : 0) | (a.link.world > 0 ? 2 : 0) | (a.B == 1 ? 1 : 0);
