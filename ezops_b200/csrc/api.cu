@@ -144,6 +144,7 @@ static size_t round256(size_t v) { return (v + 255) / 256 * 256; }
 struct LayerWorkspace {
     void* attn;
     bf16 *qkv, *attn_out, *x2, *h, *xn;
+    float* ssq;  // batch >= 2: sums of squares of the residual stream's rows (deferred norms)
     void* mega;  // batch 1: barrier counters and slice records of the single-kernel layer (zero before first use)
     size_t total;
 };
@@ -163,6 +164,7 @@ static LayerWorkspace carve_layer_ws(void* base, int B, int S, int H, int I, int
     w.x2 = reinterpret_cast<bf16*>(take((size_t)B * H * 2));
     w.h = reinterpret_cast<bf16*>(take((size_t)B * I * 2));
     w.xn = reinterpret_cast<bf16*>(take((size_t)B * H * 2));
+    w.ssq = (B > 1) ? reinterpret_cast<float*>(take(ssq_bytes(H))) : nullptr;
     w.mega = (B == 1) ? take(decode_mega_workspace_bytes(NKV, D)) : nullptr;
     w.total = off;
     return w;
@@ -170,6 +172,7 @@ static LayerWorkspace carve_layer_ws(void* base, int B, int S, int H, int I, int
 
 struct FfnWorkspace {
     bf16 *x2, *h, *xn;
+    float* ssq;
     size_t total;
 };
 
@@ -185,6 +188,7 @@ static FfnWorkspace carve_ffn_ws(void* base, int B, int H, int I) {
     w.x2 = reinterpret_cast<bf16*>(take((size_t)B * H * 2));
     w.h = reinterpret_cast<bf16*>(take((size_t)B * I * 2));
     w.xn = reinterpret_cast<bf16*>(take((size_t)B * H * 2));
+    w.ssq = (B > 1) ? reinterpret_cast<float*>(take(ssq_bytes(H))) : nullptr;
     w.total = off;
     return w;
 }
@@ -214,25 +218,40 @@ static PrefetchList one_plan(const PrefetchPlan& a) {
     return l;
 }
 
-// o_proj (+residual or fp32 partial), gate/up + SwiGLU, down (+residual or fp32 partial)
-static cudaError_t launch_o_proj(const bf16* attn, const bf16* Wo, int B, int H, int Q, const bf16* residual, void* out,
-                                 bool f32_partial, cudaStream_t stream, const PrefetchList& next = kNoPrefetch) {
+// A norm whose factor the consuming projection applies (GemvArgs::ssq): what its producer left.  `x` null: no such
+// norm, the consumer normalises by itself.
+struct DeferredNorm {
+    const bf16* x = nullptr;  // rows with the norm weight applied
+    TcTiling tiling;
+};
+
+// o_proj (+residual or fp32 partial), gate/up + SwiGLU, down (+residual or fp32 partial).  A projection with `norm`
+// prepares the norm (weight `next_norm_w`, may be null) of its result, through ssq and xw.
+static cudaError_t launch_residual_proj(int trace_id, const bf16* x, const bf16* W, int B, int N, int K, const bf16* residual, void* out,
+                                        bool f32_partial, cudaStream_t stream, const PrefetchList& next = kNoPrefetch,
+                                        DeferredNorm* norm = nullptr, const bf16* next_norm_w = nullptr, float* ssq = nullptr,
+                                        bf16* xw = nullptr) {
     GemvArgs g;
     g.allow_tc = B >= 2;
-    g.W0 = Wo, g.ldw = Q, g.N = H, g.K = Q, g.B = B;
-    g.x = attn, g.ldx = Q;
+    g.W0 = W, g.ldw = K, g.N = N, g.K = K, g.B = B;
+    g.x = x, g.ldx = K;
     g.prologue = PRO_NONE;
     g.epilogue = f32_partial ? EPI_STORE_F32 : EPI_RESIDUAL;
-    g.residual = residual, g.ldres = H;
-    g.out = out, g.ldout = H;
+    g.residual = residual, g.ldres = N;
+    g.out = out, g.ldout = N;
     g.next = next;
-    g.trace_id = 3;
+    g.trace_id = trace_id;
+    if (norm && B >= 2 && gemv_uses_tc(B, K) && gemv_uses_tc(B, N)) {
+        g.ssq = ssq, g.tiling = &norm->tiling, g.next_norm_w = next_norm_w, g.xw_out = xw;
+        norm->x = next_norm_w ? xw : static_cast<const bf16*>(out);
+    }
     return launch_gemv(g, stream);
 }
 
 static cudaError_t launch_gate_up(const bf16* x, const float* x_add, bf16* x_sum_out, const bf16* norm_w, const bf16* Wg,
                                   const bf16* Wu, int B, int H, int I, float eps, bf16* h, bf16* xn_scratch,
-                                  cudaStream_t stream, const PrefetchList& next = kNoPrefetch) {
+                                  cudaStream_t stream, const PrefetchList& next = kNoPrefetch, DeferredNorm* norm = nullptr,
+                                  float* ssq = nullptr) {
     GemvArgs g;
     g.allow_tc = B >= 2;
     g.W0 = Wg, g.W1 = Wu, g.ldw = H, g.N = I, g.K = H, g.B = B;
@@ -240,26 +259,12 @@ static cudaError_t launch_gate_up(const bf16* x, const float* x_add, bf16* x_sum
     g.x_add = x_add, g.ldadd = H, g.x_sum_out = x_sum_out, g.ldsum = H;
     g.norm_w = norm_w, g.eps = eps;
     g.prologue = x_add ? PRO_ADD_RMSNORM : PRO_RMSNORM;
+    if (norm && norm->x) g.prologue = PRO_SCALED, g.x = norm->x, g.ssq = ssq, g.tiling = &norm->tiling;
     g.epilogue = EPI_SWIGLU;
     g.out = h, g.ldout = I;
     g.xn_scratch = xn_scratch;
     g.next = next;
     g.trace_id = 4;
-    return launch_gemv(g, stream);
-}
-
-static cudaError_t launch_down(const bf16* h, const bf16* Wd, int B, int H, int I, const bf16* residual, void* out,
-                               bool f32_partial, cudaStream_t stream, const PrefetchList& next = kNoPrefetch) {
-    GemvArgs g;
-    g.allow_tc = B >= 2;
-    g.W0 = Wd, g.ldw = I, g.N = H, g.K = I, g.B = B;
-    g.x = h, g.ldx = I;
-    g.prologue = PRO_NONE;
-    g.epilogue = f32_partial ? EPI_STORE_F32 : EPI_RESIDUAL;
-    g.residual = residual, g.ldres = H;
-    g.out = out, g.ldout = H;
-    g.trace_id = 5;
-    g.next = next;
     return launch_gemv(g, stream);
 }
 
@@ -274,6 +279,7 @@ struct LayerExtras {
     const bf16* rope_cos = nullptr;
     const bf16* rope_sin = nullptr;
     const bf16* next_Wqkv = nullptr;
+    const bf16* next_input_norm_w = nullptr;  // of the layer that follows
     const int* seq_lens = nullptr;  // per-row valid lengths (device); the new token goes to slot len-1
     int rope_by_len = 0;            // rope_cos / rope_sin are table bases indexed by that slot
     const int* page_table = nullptr;  // paged caches (see AttnArgs)
@@ -284,13 +290,14 @@ static const LayerExtras kPlainLayer = {};
 static cudaError_t launch_qkv_and_attention(const bf16* hidden, bf16* Kc, bf16* Vc, const bf16* Wqkv, const LayerWorkspace& w,
                                             int B, int S, int H, int NH, int NKV, int D, float eps, cudaStream_t stream,
                                             const bf16* Wo, const PrefetchPlan* after_wo = nullptr,
-                                            const LayerExtras& ex = kPlainLayer) {
+                                            const LayerExtras& ex = kPlainLayer, DeferredNorm* norm = nullptr) {
     const int rows = (NH + 2 * NKV) * D;
     GemvArgs g;
     g.W0 = Wqkv, g.ldw = H, g.N = rows, g.K = H, g.B = B;
     g.x = hidden, g.ldx = H;
     g.norm_w = ex.input_norm_w;
     g.eps = eps, g.prologue = PRO_RMSNORM, g.epilogue = EPI_STORE;
+    if (norm && norm->x) g.prologue = PRO_SCALED, g.x = norm->x, g.ssq = w.ssq, g.tiling = &norm->tiling;
     g.out = w.qkv, g.ldout = rows;
     g.xn_scratch = w.xn;
     g.allow_tc = B >= 2;
@@ -547,13 +554,15 @@ int ezb_o_proj_ffn(const void* attn, const void* residual, const void* Wo, const
     }
     chain_begin();
     const int pf_kb = tuning(EZB_TUNE_L2_PREFETCH_KB);
-    EZB_CUDA_TRY(launch_o_proj(static_cast<const bf16*>(attn), static_cast<const bf16*>(Wo), B, H, Q,
-                               static_cast<const bf16*>(residual), w.x2, false, stream,
-                               one_plan(next_rows(static_cast<const bf16*>(Wg), static_cast<const bf16*>(Wu), I, H, pf_kb))));
+    DeferredNorm norm;
+    EZB_CUDA_TRY(launch_residual_proj(3, static_cast<const bf16*>(attn), static_cast<const bf16*>(Wo), B, H, Q,
+                                      static_cast<const bf16*>(residual), w.x2, false, stream,
+                                      one_plan(next_rows(static_cast<const bf16*>(Wg), static_cast<const bf16*>(Wu), I, H, pf_kb)), &norm,
+                                      static_cast<const bf16*>(post_norm_w), w.ssq, w.xn));
     EZB_CUDA_TRY(launch_gate_up(w.x2, nullptr, nullptr, static_cast<const bf16*>(post_norm_w), static_cast<const bf16*>(Wg),
                                 static_cast<const bf16*>(Wu), B, H, I, eps, w.h, w.xn, stream,
-                                one_plan(next_rows(static_cast<const bf16*>(Wd), nullptr, H, I, pf_kb))));
-    EZB_CUDA_TRY(launch_down(w.h, static_cast<const bf16*>(Wd), B, H, I, w.x2, out, false, stream, kNoPrefetch));
+                                one_plan(next_rows(static_cast<const bf16*>(Wd), nullptr, H, I, pf_kb)), &norm, w.ssq));
+    EZB_CUDA_TRY(launch_residual_proj(5, w.h, static_cast<const bf16*>(Wd), B, H, I, w.x2, out, false, stream));
     return EZB_OK;
 }
 
@@ -576,10 +585,12 @@ static MegaArgs mega_args(const bf16* hid, bf16* Kc, bf16* Vc, const bf16* Wqkv,
     return m;
 }
 
-// One layer's five (seven with the tensor-core path) launches.  The caller has opened the chain.
+// One layer's five launches (batch >= 2: one more in front where nobody has prepared the first norm).  The caller has
+// opened the chain.  `first`: the first norm as the previous layer of a stack left it; updated for the layer that
+// follows (ex.next_Wqkv).
 static int run_layer(const bf16* hid, bf16* Kc, bf16* Vc, const bf16* Wqkv, const bf16* Wo, const bf16* wgu, const bf16* Wd,
                      bf16* out, const LayerWorkspace& w, int B, int S, int H, int I, int NH, int NKV, int D, float eps,
-                     const LayerExtras& ex, cudaStream_t stream) {
+                     const LayerExtras& ex, cudaStream_t stream, DeferredNorm* first = nullptr) {
     if (B == 1 && !ex.seq_lens && !ex.page_table && w.mega) {
         // batch 1 on contiguous caches: the whole layer as one persistent kernel
         const MegaArgs m = mega_args(hid, Kc, Vc, Wqkv, Wo, wgu, Wd, out, w, S, H, I, NH, NKV, D, eps, ex);
@@ -593,13 +604,17 @@ static int run_layer(const bf16* hid, bf16* Kc, bf16* Vc, const bf16* Wqkv, cons
     // attention is latency-bound: besides Wo it can pull the head of the gate/up rows; o_proj then pulls the rows after those
     const PrefetchPlan gu_head = next_rows(wgu, wgu + (size_t)I * H, I, H, pf_attn_kb);
     EZB_CUDA_TRY(launch_qkv_and_attention(hid, Kc, Vc, Wqkv, w, B, S, H, NH, NKV, D, eps, stream, Wo,
-                                          pf_attn_kb > 0 ? &gu_head : nullptr, ex));
-    EZB_CUDA_TRY(launch_o_proj(w.attn_out, Wo, B, H, NH * D, hid, w.x2, false, stream,
-                               one_plan(next_rows(wgu, wgu + (size_t)I * H, I, H, pf_kb, pf_attn_kb > 0 ? pf_attn_kb : 0))));
+                                          pf_attn_kb > 0 ? &gu_head : nullptr, ex, first));
+    DeferredNorm post;
+    EZB_CUDA_TRY(launch_residual_proj(3, w.attn_out, Wo, B, H, NH * D, hid, w.x2, false, stream,
+                                      one_plan(next_rows(wgu, wgu + (size_t)I * H, I, H, pf_kb, pf_attn_kb > 0 ? pf_attn_kb : 0)), &post,
+                                      ex.post_norm_w, w.ssq, w.xn));
     EZB_CUDA_TRY(launch_gate_up(w.x2, nullptr, nullptr, ex.post_norm_w, wgu, wgu + (size_t)I * H, B, H, I, eps, w.h, w.xn, stream,
-                                one_plan(next_rows(Wd, nullptr, H, I, pf_kb))));
+                                one_plan(next_rows(Wd, nullptr, H, I, pf_kb)), &post, w.ssq));
     const PrefetchList after = ex.next_Wqkv ? one_plan(next_rows(ex.next_Wqkv, nullptr, (NH + 2 * NKV) * D, H, pf_kb)) : kNoPrefetch;
-    EZB_CUDA_TRY(launch_down(w.h, Wd, B, H, I, w.x2, out, false, stream, after));
+    if (first) first->x = nullptr;
+    EZB_CUDA_TRY(launch_residual_proj(5, w.h, Wd, B, H, I, w.x2, out, false, stream, after, ex.next_Wqkv ? first : nullptr,
+                                      ex.next_input_norm_w, w.ssq, w.xn));
     return EZB_OK;
 }
 
@@ -658,19 +673,21 @@ static int run_stack(const void* hidden, void* out, const ezb_layer_t* layers, i
     const bf16* sin_row = rope_sin ? static_cast<const bf16*>(rope_sin) + row_off : nullptr;
     chain_begin();  // one dependency chain through all layers
     const bf16* x = static_cast<const bf16*>(hidden);
+    DeferredNorm norm;
     for (int l = 0; l < n_layers; ++l) {
         const ezb_layer_t& L = layers[l];
         LayerExtras ex;
         ex.input_norm_w = static_cast<const bf16*>(L.input_norm_w), ex.post_norm_w = static_cast<const bf16*>(L.post_norm_w);
         ex.q_norm_w = static_cast<const bf16*>(L.q_norm_w), ex.k_norm_w = static_cast<const bf16*>(L.k_norm_w);
         ex.rope_cos = cos_row, ex.rope_sin = sin_row;
+        ex.next_input_norm_w = (l + 1 < n_layers) ? static_cast<const bf16*>(layers[l + 1].input_norm_w) : nullptr;
         ex.seq_lens = seq_lens, ex.rope_by_len = seq_lens ? 1 : 0;
         ex.page_table = page_table, ex.page_shift = page_shift, ex.max_pages = max_pages, ex.num_pages = num_pages;
         ex.next_Wqkv = (l + 1 < n_layers) ? static_cast<const bf16*>(layers[l + 1].Wqkv) : nullptr;
         bf16* y = (l + 1 == n_layers) ? static_cast<bf16*>(out) : pp[l & 1];
         if (int rc = run_layer(x, static_cast<bf16*>(L.K_cache), static_cast<bf16*>(L.V_cache), static_cast<const bf16*>(L.Wqkv),
                                static_cast<const bf16*>(L.Wo), static_cast<const bf16*>(L.Wgu), static_cast<const bf16*>(L.Wd), y,
-                               w, B, S, H, I, NH, NKV, D, eps, ex, static_cast<cudaStream_t>(stream)))
+                               w, B, S, H, I, NH, NKV, D, eps, ex, static_cast<cudaStream_t>(stream), &norm))
             return rc;
         x = y;
     }
@@ -696,8 +713,8 @@ int ezb_qwen3_decode_layer_tp_attn(const void* hidden, void* K_cache, void* V_ca
     EZB_CUDA_TRY(launch_qkv_and_attention(static_cast<const bf16*>(hidden), static_cast<bf16*>(K_cache),
                                           static_cast<bf16*>(V_cache), static_cast<const bf16*>(Wqkv_local), w, B, S, H,
                                           NH_local, NKV_local, D, eps, stream, static_cast<const bf16*>(Wo_local)));
-    EZB_CUDA_TRY(launch_o_proj(w.attn_out, static_cast<const bf16*>(Wo_local), B, H, NH_local * D, nullptr, partial_o, true,
-                               stream, kNoPrefetch));
+    EZB_CUDA_TRY(launch_residual_proj(3, w.attn_out, static_cast<const bf16*>(Wo_local), B, H, NH_local * D, nullptr, partial_o, true,
+                                      stream));
     return EZB_OK;
 }
 
@@ -719,8 +736,7 @@ int ezb_qwen3_decode_layer_tp_ffn(const void* hidden, const float* summed_o, con
     EZB_CUDA_TRY(launch_gate_up(static_cast<const bf16*>(hidden), summed_o, static_cast<bf16*>(x2), nullptr, wgu,
                                 wgu + (size_t)I_local * H, B, H, I_local, eps, w.h, w.xn, stream,
                                 one_plan(next_rows(static_cast<const bf16*>(Wd_local), nullptr, H, I_local, tuning(EZB_TUNE_L2_PREFETCH_KB)))));
-    EZB_CUDA_TRY(launch_down(w.h, static_cast<const bf16*>(Wd_local), B, H, I_local, nullptr, partial_d, true, stream,
-                             kNoPrefetch));
+    EZB_CUDA_TRY(launch_residual_proj(5, w.h, static_cast<const bf16*>(Wd_local), B, H, I_local, nullptr, partial_d, true, stream));
     return EZB_OK;
 }
 
@@ -902,8 +918,12 @@ static int check_tp_fused_shape(int B, int H, int I_local, int NH_local, int NKV
 static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_in, bf16* x2_out, bf16* Kc, bf16* Vc,
                               const bf16* Wqkv, const bf16* Wo, const bf16* wgu, const bf16* Wd, const LayerWorkspace& w,
                               const TpLink& base, int B, int S, int H, int I_local, int NH_local, int NKV_local, int D, float eps,
-                              const LayerExtras& ex, cudaStream_t stream) {
+                              const LayerExtras& ex, cudaStream_t stream, TcTiling& down_tiling) {
     const int Q = NH_local * D, rows = (NH_local + 2 * NKV_local) * D;
+    // batch >= 2: the row kernel that gathers a sum leaves the norm to the projection behind it, in the form (and with
+    // the bits) in which the single-GPU chain's projections leave it; `down_tiling` is the previous layer's
+    float* ssq = (B >= 2 && gemv_uses_tc(B, H) && gemv_uses_tc(B, Q) && gemv_uses_tc(B, I_local)) ? w.ssq : nullptr;
+    TcTiling o_tiling;
     const int pf_kb = tuning(EZB_TUNE_L2_PREFETCH_KB);
     const bf16* hid = gather_prev ? layer_in : x_prev;
     {   // QKV projection (norm prologue; gathers the previous layer's second sum when there is one)
@@ -918,6 +938,7 @@ static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_
         if (gather_prev) {
             g.x_sum_out = layer_in, g.ldsum = H;
             g.link = base, g.link.gather_inbox = 1;
+            g.ssq = ssq, g.tiling = &down_tiling;
         }
         const size_t kv_bytes = (size_t)B * NKV_local * S * D * 2;
         if (2 * kv_bytes <= ((size_t)48 << 20)) g.next = one_plan(prefetch_plan_flat(Kc, Vc, kv_bytes));
@@ -945,6 +966,7 @@ static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_
         g.x = w.attn_out, g.ldx = Q;
         g.epilogue = EPI_PUSH_F32, g.ldout = H;
         g.link = base, g.link.push_inbox = 0, g.link.bump_inbox = 1;
+        g.tiling = &o_tiling;
         g.next = one_plan(next_rows(wgu, wgu + (size_t)I_local * H, I_local, H, pf_kb));
         g.trace_id = 3;
         EZB_CUDA_TRY(launch_gemv(g, stream));
@@ -959,6 +981,7 @@ static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_
         g.eps = eps, g.prologue = PRO_ADD_RMSNORM, g.epilogue = EPI_SWIGLU;
         g.out = w.h, g.ldout = I_local;
         g.link = base, g.link.gather_inbox = 0;
+        g.ssq = ssq, g.tiling = &o_tiling;
         g.next = one_plan(next_rows(Wd, nullptr, H, I_local, pf_kb));
         g.trace_id = 4;
         EZB_CUDA_TRY(launch_gemv(g, stream));
@@ -970,6 +993,7 @@ static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_
         g.x = w.h, g.ldx = I_local;
         g.epilogue = EPI_PUSH_F32, g.ldout = H;
         g.link = base, g.link.push_inbox = 1, g.link.bump_inbox = 0;
+        g.tiling = &down_tiling;
         if (ex.next_Wqkv) g.next = one_plan(next_rows(ex.next_Wqkv, nullptr, rows, H, pf_kb));
         g.trace_id = 5;
         EZB_CUDA_TRY(launch_gemv(g, stream));
@@ -1020,11 +1044,12 @@ int ezb_qwen3_decode_layer_tp_fused(const void* hidden, void* K_cache, void* V_c
             return EZB_OK;
         }
     }
+    TcTiling down_tiling;
     if (int rc = run_layer_tp_fused(static_cast<const bf16*>(hidden), false, nullptr, w.x2, static_cast<bf16*>(K_cache),
                                     static_cast<bf16*>(V_cache), static_cast<const bf16*>(Wqkv_local),
                                     static_cast<const bf16*>(Wo_local), static_cast<const bf16*>(Wgu_local),
                                     static_cast<const bf16*>(Wd_local), w, base, B, S, H, I_local, NH_local, NKV_local, D, eps,
-                                    kPlainLayer, st))
+                                    kPlainLayer, st, down_tiling))
         return rc;
     return finish_tp_fused(w.x2, static_cast<bf16*>(out), base, B, H, st);
 }
@@ -1088,6 +1113,7 @@ int ezb_qwen3_decode_stack_tp_fused(const void* hidden, void* out, const ezb_lay
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     chain_begin();
     bool single_kernel = B == 1 && !seq_lens && w.mega;
+    TcTiling down_tiling;
     for (int l = 0; l < n_layers; ++l) {
         const ezb_layer_t& L = layers_local[l];
         LayerExtras ex;
@@ -1116,7 +1142,7 @@ int ezb_qwen3_decode_stack_tp_fused(const void* hidden, void* out, const ezb_lay
         if (int rc = run_layer_tp_fused(x_prev, l > 0, layer_in[l & 1], x2[l & 1], static_cast<bf16*>(L.K_cache),
                                         static_cast<bf16*>(L.V_cache), static_cast<const bf16*>(L.Wqkv),
                                         static_cast<const bf16*>(L.Wo), static_cast<const bf16*>(L.Wgu),
-                                        static_cast<const bf16*>(L.Wd), w, base, B, S, H, I_local, NH_local, NKV_local, D, eps, ex, st))
+                                        static_cast<const bf16*>(L.Wd), w, base, B, S, H, I_local, NH_local, NKV_local, D, eps, ex, st, down_tiling))
             return rc;
     }
     return finish_tp_fused(x2[(n_layers - 1) & 1], static_cast<bf16*>(out), base, B, H, st);

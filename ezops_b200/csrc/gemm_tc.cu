@@ -37,7 +37,8 @@ static constexpr int kTcEpiWarps = 8;
 static constexpr int kTcThreads = 64 + 32 * kTcEpiWarps;  // TMA warp, MMA warp, epilogue warps
 static constexpr int kTcMaxStages = 40;
 static constexpr int kTcMaxCluster = 8;
-static constexpr int kTcTailBytes = 1024;  // barriers, tensor-memory slot, abort flag
+static constexpr int kTcNormAt = 1024;     // scratch of the norm factors behind the barriers: 256 partial sums, 64 factors
+static constexpr int kTcTailBytes = kTcNormAt + (256 + 64) * 4;
 
 struct TcParams {
     int N, K, B;          // output units (rows, or gate/up pairs), reduction length, batch
@@ -55,6 +56,14 @@ struct TcParams {
     void* out;
     long long ldout;
     unsigned int* status;
+    // deferred RMSNorm (GemvArgs::ssq)
+    const float* ssq_in;  // sums of squares of the input rows; their factor is applied to the products
+    int ssq_parts;
+    float inv_dim, eps;
+    int cols_pad;       // cpc rounded up to a power of two
+    float* ssq_out;     // sums of squares of the result rows, one part per tile and 32 rows
+    bf16* xw_out;       // result * next_norm_w
+    const bf16* next_norm_w;
     Trace trace;
     int trace_id;
     TpLink link;  // fused tensor-parallel exchange (world 0: none); only the push side lives in this kernel
@@ -126,7 +135,9 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+// Relaxed: what the peers must see first is ordered otherwise (fence.mbarrier_init at the start; at the end every copy
+// and arrival towards a peer has been waited for by that peer).  The release form waited for every store in flight.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 // Address of `local` (a shared::cta address) in the shared memory of cluster CTA `rank`.
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
@@ -192,6 +203,9 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 // What bounds it: the weight stream.  A tile's parts meet in shared memory because the round trips of a reduction
 // through L2 (park, ticket, read 4..19 parts in one CTA) cost 5..13 us at the end of every projection.
 // Measured: Qwen3-8B layer, batch 32, KV 4096 187.9 -> 168.0 us; eight 2B layers, batch 13, paged 680 -> 488 us.
+// A norm in front of a projection is left to its epilogue (ssq_in): the kernel that produced the rows has written their
+// sums of squares and the rows times the norm weight, so no row kernel runs between two projections (3..6 us each; the
+// 2B layers above 488 -> 438 us, 28 layers of 0.6B at batch 4 928 -> 858 us).
 // LINK: the instance whose epilogue pushes its fp32 results into the peers' inboxes (see TpLink).
 template <int NB, bool LINK>
 __global__ void __launch_bounds__(kTcThreads, 2)
@@ -216,6 +230,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant_
     uint64_t* recv_free = recv_full + 1;            // all CTAs of the cluster have read what this CTA sent them
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(recv_free + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    float* norm_sum = reinterpret_cast<float*>(tail + kTcNormAt);                // [256 / cols_pad][cols_pad]
+    float* norm_r = norm_sum + 256;                                             // norm factor of each column of this CTA
     const int RS = p.a_rows;                                                    // rows of a column of a partial tile
     float* mine = reinterpret_cast<float*>(tail + kTcTailBytes);                // [column][RS]: this CTA's part of the tile
     float* recv = mine + (size_t)(p.cpc << p.log2c) * RS;                       // [sender][column of this CTA][RS]
@@ -357,6 +373,25 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant_
         trace_mark(trec, 3);
         const unsigned int push_epoch = (LINK && p.link.world > 0 && p.link.push_inbox >= 0) ? tp_next_epoch(p.link, p.link.push_inbox) : 0u;
         const bool poisoned = LINK && p.link.world > 0 && tp_poisoned(p.status);  // see tp_poisoned: push nothing, advance nothing
+        if (p.ssq_in) {
+            // The norm factors of this CTA's columns, from the parts that the kernel in front left (fixed order), while
+            // the products are being formed.
+            const int c = et & (p.cols_pad - 1), j0 = et / p.cols_pad, per_col = 32 * kTcEpiWarps / p.cols_pad;
+            float sum = 0.f;
+            if (c < n_cols) {
+                const float* src = p.ssq_in + b_first + c;
+#pragma unroll 4
+                for (int j = j0; j < p.ssq_parts; j += per_col) sum += __ldcg(src + (long long)j * kSsqStride);
+            }
+            norm_sum[c * per_col + j0] = sum;
+            named_bar_sync(2, 32 * kTcEpiWarps);
+            if (et < n_cols) {
+                float tot = 0.f;
+                for (int j = 0; j < per_col; ++j) tot += norm_sum[et * per_col + j];
+                norm_r[et] = 1.0f / sqrtf(tot * p.inv_dim + p.eps);
+            }
+            named_bar_sync(2, 32 * kTcEpiWarps);
+        }
         for (int i = 0; i < my_tiles; ++i) {
             const int tile = cluster + i * n_clusters;
             const int acc = i & 1;
@@ -374,6 +409,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant_
                 }
             };
             if (p.epilogue == EPI_RESIDUAL && live_row) fetch_residual(cg);
+            const float next_w = (p.xw_out && live_row) ? __bfloat162float(p.next_norm_w[n]) : 0.f;
             mbar_wait_bounded(smem_u32(&acc_full[acc]), (uint32_t)((i >> 1) & 1), abort_flag, p.status, FAULT_TC_ACC_WAIT);
             if (i == 0) trace_mark(trec, 4);
             tc_fence_after();
@@ -429,8 +465,40 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant_
                     for (int u = 0; u < CU; ++u)
                         if (col + u * groups < n_cols) v[u] += part[u * groups * RS];
                 }
+                if (p.ssq_in) {
+#pragma unroll
+                    for (int u = 0; u < CU; ++u)
+                        if (col + u * groups < n_cols) v[u] *= norm_r[col + u * groups];
+                }
             };
-            if (!*abort_flag && live_row) {
+            if (p.ssq_out) {
+                // Residual epilogue in front of a norm: the result, the result with the norm weight, and the sum of
+                // squares of the warp's 32 rows of each column.
+                const int q32 = (et & 127) >> 5, q32s = (p.units + 31) >> 5;
+                if (!*abort_flag && q32 < q32s) {
+                    for (int col = cg; col < n_cols; col += CU * groups) {
+                        float v[CU];
+                        gather(col, min(frow, RS - 1), v);
+                        if (col != cg && live_row) fetch_residual(col);
+#pragma unroll
+                        for (int u = 0; u < CU; ++u) {
+                            const int c = col + u * groups;
+                            if (c < n_cols) {
+                                float x = 0.f;
+                                if (live_row) {
+                                    const bf16 xb = __float2bfloat16_rn(res[u] + round_bf16(v[u]));
+                                    x = __bfloat162float(xb);
+                                    const long long o = (long long)(b_first + c) * p.ldout + n;
+                                    reinterpret_cast<bf16*>(p.out)[o] = xb;
+                                    if (p.xw_out) p.xw_out[(long long)(b_first + c) * p.N + n] = __float2bfloat16_rn(x * next_w);
+                                }
+                                const float sum = warp_sum(x * x);
+                                if (lane == 0) p.ssq_out[(long long)(tile * q32s + q32) * kSsqStride + b_first + c] = sum;
+                            }
+                        }
+                    }
+                }
+            } else if (!*abort_flag && live_row) {
                 float v[CU];
                 const long long step = (long long)groups * p.ldout;
                 for (int col = cg; col < n_cols; col += CU * groups) {
@@ -604,7 +672,7 @@ static int tc_resident_clusters(int dev, int log2c, bool half) {
 // fitted to a sweep of every projection over all cluster sizes (Qwen3 0.6B / 2B / 8B / 32B, batch 2..64; e.g. 8B at batch
 // 32, layer us with clusters of 1 | 2 | 4 | 8: gate/up 174.5 | 168.9 | 171.1 | 185.1, down 191.4 | 175.0 | 171.0 | 172.3;
 // 0.6B o_proj 64.9 | 60.5 | 58.6 | 58.4).  A k-block costs 40 ns plus its bytes at a 148th of the HBM rate (never less
-// than 95 ns: the MMAs read 128 rows of A from shared memory whatever the tile holds).
+// than 150 ns: waiting for a stage and issuing its MMAs, which read 128 rows of A whatever the tile holds).
 template <int NB, bool LINK>
 static bool tc_plan(TcParams& p, int dev, int& clusters, size_t& smem) {
     double best = 0.;
@@ -633,7 +701,7 @@ static bool tc_plan(TcParams& p, int dev, int& clusters, size_t& smem) {
             if (all) ns = rounds * nk < 2 ? 2 : rounds * nk;
             if (half && !all) continue;  // a long stream wants the deeper ring
             const double block = 40. + 2.6 * (p.pair ? 2 * units : units) + 0.9 * NB;
-            const double tile = nk * (block < 95. ? 95. : block), epi = (C > 1 ? 1500. : 500.) + 60. * cpc;
+            const double tile = nk * (block < 150. ? 150. : block), epi = (C > 1 ? 1100. : 800.) + 60. * cpc;
             const double cost = rounds * tile + (rounds - 1) * (epi > tile ? epi - tile : 0.) + epi;
             if (best > 0. && cost >= best) continue;
             best = cost;
@@ -660,6 +728,9 @@ static cudaError_t launch_tc_instance(const GemvArgs& a, const bf16* x, long lon
     int clusters = 0;
     size_t smem = 0;
     if (!tc_plan<NB, LINK>(p, dev, clusters, smem)) return cudaErrorInvalidConfiguration;
+    if (a.tiling && a.prologue != PRO_SCALED) a.tiling->units = p.units, a.tiling->tiles = p.tiles;
+    p.cols_pad = 1;
+    while (p.cols_pad < p.cpc) p.cols_pad *= 2;
     alignas(64) CUtensorMap m0, m1, mx;
     if (!make_map(&m0, a.W0, a.N, a.K, a.ldw, p.units)) return cudaErrorInvalidValue;
     if (!make_map(&m1, p.pair ? a.W1 : a.W0, a.N, a.K, a.ldw, p.units)) return cudaErrorInvalidValue;
@@ -667,7 +738,7 @@ static cudaError_t launch_tc_instance(const GemvArgs& a, const bf16* x, long lon
     return launch_pdl_cluster(kernel, dim3((unsigned)clusters << p.log2c), dim3(kTcThreads), 1 << p.log2c, smem, stream, m0, m1, mx, p);
 }
 
-// x must already hold what the MMA consumes (any norm prologue has been run by the caller).
+// x must already hold what the MMA consumes; the prologue is none or PRO_SCALED.
 cudaError_t launch_gemm_tc(const GemvArgs& a, const bf16* x, long long ldx, cudaStream_t stream) {
     const bool pair = a.epilogue == EPI_SWIGLU;
     TcParams p;
@@ -681,6 +752,10 @@ cudaError_t launch_gemm_tc(const GemvArgs& a, const bf16* x, long long ldx, cuda
     if (!p.status) return cudaErrorUnknown;
     p.trace = trace_handle();
     p.trace_id = a.trace_id;
+    p.ssq_in = nullptr, p.ssq_parts = 0, p.inv_dim = 1.0f / (float)a.K, p.eps = a.eps;
+    p.ssq_out = nullptr, p.xw_out = nullptr, p.next_norm_w = a.next_norm_w;
+    if (a.prologue == PRO_SCALED) p.ssq_in = a.ssq, p.ssq_parts = a.tiling->parts();
+    else if (a.ssq && a.epilogue == EPI_RESIDUAL) p.ssq_out = a.ssq, p.xw_out = a.next_norm_w ? a.xw_out : nullptr;
     p.link = a.link;
     if (a.link.world > 0 && (a.link.gather_inbox >= 0 || pair)) return cudaErrorNotSupported;  // only the push side lives here
     const int NB = tc_batch_tile(a.B);

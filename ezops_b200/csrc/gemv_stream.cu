@@ -863,6 +863,10 @@ static bool plan_rows8(const GemvArgs& a, GemvPlan& pl) {
     return true;
 }
 
+// Two rows and more go to the tensor cores: staging the rows in every CTA of the small-batch kernel costs 3 us at 2 rows
+// and 8 us at 8 (Qwen3-8B layer, KV 4096, batch 8: 120 us with it, 104 us without; batch 2: 94 and 89 us).
+bool gemv_uses_tc(int B, int K) { return tuning(EZB_TUNE_TC) != 0 && gemm_tc_supported(B, K); }
+
 bool gemv_small_batch_eligible(int B, int K) {
     if (tuning(EZB_TUNE_GEMV_ROWS8) == 0) return false;
     GemvArgs a;
@@ -888,7 +892,8 @@ static cudaError_t launch_rows8(const GemvParams& p, const GemvPlan& pl, cudaStr
 cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream) {
     const bool pair = a.epilogue == EPI_SWIGLU;
     GemvPlan pl;
-    const bool rows8 = tuning(EZB_TUNE_GEMV_ROWS8) != 0 && plan_rows8(a, pl);
+    const bool use_tc = a.allow_tc && gemv_uses_tc(a.B, a.K);
+    const bool rows8 = !use_tc && tuning(EZB_TUNE_GEMV_ROWS8) != 0 && plan_rows8(a, pl);
     if (!rows8) pl = plan_gemv(a, pair);
 
     GemvParams p;
@@ -912,14 +917,13 @@ cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream) {
     p.trace_id = a.trace_id;
     p.link = a.link;
 
-    const bool use_tc = !rows8 && a.allow_tc && tuning(EZB_TUNE_TC) != 0 && gemm_tc_supported(a.B, a.K);
-    // The fused tensor-parallel exchange lives in the small-batch kernel (gather and push) and, for larger
-    // batches, in the row kernel (gather) and the tensor-core kernel (push); the general fallback has none.
+    // The fused tensor-parallel exchange lives in the row kernel (gather) and the tensor-core kernel (push) and, at
+    // batch 1, in the small-batch kernel (both); the general fallback has none.
     const bool linked = a.link.world > 0;
     const bool gathers = linked && a.link.gather_inbox >= 0;
     if (linked && !rows8 && !use_tc) return cudaErrorNotSupported;
     GemvArgs tc_args = a;
-    if ((use_tc || !pl.xres) && a.prologue != PRO_NONE) {
+    if ((use_tc || !pl.xres) && a.prologue != PRO_NONE && a.prologue != PRO_SCALED) {
         // The activation block is not resident in this path: run the prologue as
         // its own (tiny) kernel into the scratch rows, then stream those.
         RowPrepArgs rp;
@@ -934,10 +938,16 @@ cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream) {
         rp.w = a.norm_w;
         rp.y = a.xn_scratch, rp.ldy = a.K;
         rp.rows = a.B, rp.dim = a.K, rp.eps = a.eps, rp.normalize = 1;
+        const bool defer = use_tc && gathers && a.ssq;  // as the single-GPU chain does it, so that the bits agree
+        if (defer) {
+            rp.ssq = a.ssq, rp.tiling = *a.tiling;
+            if (!a.norm_w) rp.y = nullptr;
+        }
         cudaError_t e = launch_row_prep(rp, stream);
         if (e != cudaSuccess) return e;
         p.x = a.xn_scratch, p.ldx = a.K;
-        p.prologue = PRO_NONE;
+        p.prologue = tc_args.prologue = defer ? PRO_SCALED : PRO_NONE;
+        if (defer && !a.norm_w) p.x = a.x_sum_out, p.ldx = a.ldsum;
     }
     if (use_tc) return launch_gemm_tc(tc_args, p.x, p.ldx, stream);
 

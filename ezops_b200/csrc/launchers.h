@@ -12,6 +12,7 @@ enum GemvPrologue : int {
     PRO_NONE = 0,         // x is used as given
     PRO_RMSNORM = 1,      // x <- bf16(x * rsqrt(mean(x^2)+eps) [* w])
     PRO_ADD_RMSNORM = 2,  // s = bf16(x + bf16(x_add)); CTA 0 stores s; x <- rmsnorm(s)
+    PRO_SCALED = 3,       // x carries the norm weight already; its rows' norm factor is applied to the products (ssq)
 };
 enum GemvEpilogue : int {
     EPI_STORE = 0,      // out = bf16(acc)
@@ -20,6 +21,17 @@ enum GemvEpilogue : int {
     EPI_STORE_F32 = 3,  // out = acc (fp32)
     EPI_PUSH_F32 = 4,   // acc (fp32) stored into this rank's slot of an inbox on every rank (see TpLink)
 };
+
+// How a tensor-core projection dealt its output rows out: the order in which the sums of squares of its result were
+// taken (one part per tile and group of 32 rows).
+struct TcTiling {
+    int units = 0, tiles = 0;  // rows per tile, tiles
+    __host__ __device__ int groups() const { return (units + 31) / 32; }
+    __host__ __device__ int parts() const { return tiles * groups(); }
+};
+static constexpr int kSsqStride = 64;  // floats between the parts: [part][batch row]
+// Parts a projection with N output rows can produce at most (tiles have at least 8 rows, see tc_plan).
+inline size_t ssq_bytes(int N) { return ((size_t)N / 8 + 8) * kSsqStride * sizeof(float); }
 
 struct GemvArgs {
     const bf16* W0 = nullptr;  // [N, ldw]: row n produces output n (gate rows when W1 is set)
@@ -44,12 +56,21 @@ struct GemvArgs {
     PrefetchList next = {};  // what the following kernels stream first (optional)
     int trace_id = 0;  // label in timeline traces
     bool allow_tc = false;  // batch >= 2: the tensor-core path may be taken
+    // RMSNorm of this projection's result (EPI_RESIDUAL, EPI_PUSH_F32) or of its input (PRO_SCALED, PRO_ADD_RMSNORM
+    // of a gathering kernel), tensor-core path only.  The producer stores bf16(result * next_norm_w) in xw_out (when
+    // there is a weight) and the sums of squares of the result's rows, and says in `tiling` how they are cut; the
+    // consumer multiplies its products by 1 / sqrt(mean + eps).
+    float* ssq = nullptr;
+    TcTiling* tiling = nullptr;
+    const bf16* next_norm_w = nullptr;
+    bf16* xw_out = nullptr;
     TpLink link = {0, 0, {}, {}, 0, -1, -1, -1};  // fused tensor-parallel exchange (small-batch kernel only)
 };
 bool gemv_small_batch_eligible(int B, int K);  // true when launch_gemv would run the small-batch kernel
 
 // Tensor-core (tcgen05) path for batched projections, see gemm_tc.cu.
 bool gemm_tc_supported(int B, int K);
+bool gemv_uses_tc(int B, int K);  // the path launch_gemv takes when allow_tc is set
 cudaError_t launch_gemm_tc(const GemvArgs& a, const bf16* x, long long ldx, cudaStream_t stream);
 
 // Prefetch descriptors for the operands of a following kernel.
@@ -77,6 +98,10 @@ struct RowPrepArgs {
     int rows = 0, dim = 0;
     float eps = 1e-6f;
     int normalize = 1;
+    // deferred norm (see GemvArgs::ssq; needs sum_out): y = bf16(s * w) without the norm factor, sums of squares of s in
+    // the parts that a projection with this tiling would have written
+    float* ssq = nullptr;
+    TcTiling tiling;
     TpLink link = {0, 0, {}, {}, 0, -1, -1, -1};  // gather_inbox >= 0: `add` is the sum of that inbox's slots
 };
 cudaError_t launch_row_prep(const RowPrepArgs& a, cudaStream_t stream);

@@ -83,14 +83,19 @@ struct RowPrepParams {
     int dim;
     float eps;
     int normalize;
+    float* ssq;
+    TcTiling tiling;
     TpLink link;
     unsigned int* status;
 };
 
+// LINK: the instance that gathers from an inbox (its polling loop holds 64 cells in registers; the plain instance must
+// stay small, so that it shares its SMs with the projection behind it).
 // `ok` turns false (and stays false) when the wait for the peers' partials ran out: the caller then stores nothing.
+template <bool LINK>
 __device__ __forceinline__ uint4 load_row8(const RowPrepParams& p, long long row, int i, unsigned int epoch, long long t0, bool& ok) {
     uint4 raw = *reinterpret_cast<const uint4*>(p.x + row * p.ldx + i * 8);
-    if (p.link.world > 0 && p.link.gather_inbox >= 0) {
+    if (LINK && p.link.world > 0 && p.link.gather_inbox >= 0) {
         // the term to add is the sum, in rank order, of the partials in this rank's inbox
         float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         ok = ok && tp_gather<8, 8>(p.link, epoch, row * p.dim + i * 8, a, p.status, t0);
@@ -130,41 +135,64 @@ cudaError_t launch_pinned_copy(void* dst, const void* src, size_t bytes, bool to
                       n16, to_host ? 1 : 0);
 }
 
+template <bool LINK>
 __global__ void __launch_bounds__(kRowThreads) row_prep_kernel(const RowPrepParams p) {
     __shared__ float scratch[8];
     pdl_trigger();
     pdl_wait();
-    const bool gather = p.link.world > 0 && p.link.gather_inbox >= 0;
+    const bool gather = LINK && p.link.world > 0 && p.link.gather_inbox >= 0;
     if (gather && tp_poisoned(p.status)) return;  // see tp_poisoned: the chain already gave up a wait
     const unsigned int epoch = gather ? tp_next_epoch(p.link, p.link.gather_inbox) : 0u;
     const long long t0 = clock64();
     const long long row = blockIdx.x;
     const int nvec = p.dim / 8;
+    // The first kKeep vectors of a thread stay in registers between the passes (rows of up to 8192 elements entirely):
+    // the second pass then costs no further round trip, and the weights are requested together with the row.
+    constexpr int kKeep = 4;
+    uint4 keep[kKeep], wkeep[kKeep];
+    const bool weighted = p.w && p.y;
+#pragma unroll
+    for (int u = 0; u < kKeep; ++u) {
+        const int i = threadIdx.x + u * kRowThreads;
+        if (weighted && i < nvec) wkeep[u] = *reinterpret_cast<const uint4*>(p.w + i * 8);
+    }
     float ssq = 0.f;
     bool ok = true;
-    for (int i = threadIdx.x; i < nvec; i += kRowThreads) {
-        const uint4 s = load_row8(p, row, i, epoch, t0, ok);
+    auto first_pass = [&](int i) {
+        const uint4 s = load_row8<LINK>(p, row, i, epoch, t0, ok);
         if (ok && p.sum_out) *reinterpret_cast<uint4*>(p.sum_out + row * p.ldsum + i * 8) = s;
         const uint32_t w[4] = {s.x, s.y, s.z, s.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) ssq += bf16_lo(w[e]) * bf16_lo(w[e]) + bf16_hi(w[e]) * bf16_hi(w[e]);
+        return s;
+    };
+#pragma unroll
+    for (int u = 0; u < kKeep; ++u) {
+        const int i = threadIdx.x + u * kRowThreads;
+        if (i < nvec) keep[u] = first_pass(i);
+    }
+    for (int i = threadIdx.x + kKeep * kRowThreads; i < nvec; i += kRowThreads) first_pass(i);
+    if (p.ssq) {
+        // Deferred norm: the sums of squares in the parts, and in the order, of the projection whose result this is.
+        __syncthreads();
+        const int lane = threadIdx.x & 31, groups = p.tiling.groups(), parts = p.tiling.parts();
+        for (int q = threadIdx.x >> 5; q < parts; q += kRowThreads / 32) {
+            const int in_tile = (q % groups) * 32 + lane, n = (q / groups) * p.tiling.units + in_tile;
+            const float v = (in_tile < p.tiling.units && n < p.dim) ? __bfloat162float(p.sum_out[row * p.ldsum + n]) : 0.f;
+            const float sum = warp_sum(v * v);
+            if (lane == 0 && ok) p.ssq[(long long)q * kSsqStride + row] = sum;
+        }
     }
     if (!p.y) return;
     float r = 1.f;
-    if (p.normalize) {
+    if (p.normalize && !p.ssq) {
         const float tot = block_sum_256(ssq, scratch);
         r = 1.0f / sqrtf(tot / (float)p.dim + p.eps);
     }
-    for (int i = threadIdx.x; i < nvec; i += kRowThreads) {
-        const uint4 s = load_row8(p, row, i, epoch, t0, ok);
-        if (!ok) continue;
+    auto second_pass = [&](int i, const uint4& s, const uint4& q) {
         uint32_t v[4] = {s.x, s.y, s.z, s.w};
-        if (p.normalize) {
-            uint32_t nw[4] = {0, 0, 0, 0};
-            if (p.w) {
-                const uint4 q = *reinterpret_cast<const uint4*>(p.w + i * 8);
-                nw[0] = q.x, nw[1] = q.y, nw[2] = q.z, nw[3] = q.w;
-            }
+        if (p.normalize || p.ssq) {
+            const uint32_t nw[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 float lo = bf16_lo(v[e]) * r, hi = bf16_hi(v[e]) * r;
@@ -173,6 +201,18 @@ __global__ void __launch_bounds__(kRowThreads) row_prep_kernel(const RowPrepPara
             }
         }
         *reinterpret_cast<uint4*>(p.y + row * p.ldy + i * 8) = make_uint4(v[0], v[1], v[2], v[3]);
+    };
+    if (ok) {
+#pragma unroll
+        for (int u = 0; u < kKeep; ++u) {
+            const int i = threadIdx.x + u * kRowThreads;
+            if (i < nvec) second_pass(i, keep[u], wkeep[u]);
+        }
+    }
+    for (int i = threadIdx.x + kKeep * kRowThreads; i < nvec; i += kRowThreads) {
+        const uint4 s = load_row8<LINK>(p, row, i, epoch, t0, ok);
+        if (!ok) continue;
+        second_pass(i, s, weighted ? *reinterpret_cast<const uint4*>(p.w + i * 8) : make_uint4(0u, 0u, 0u, 0u));
     }
 }
 
@@ -181,10 +221,11 @@ cudaError_t launch_row_prep(const RowPrepArgs& a, cudaStream_t stream) {
     p.x = a.x, p.ldx = a.ldx, p.add = a.add, p.ldadd = a.ldadd;
     p.sum_out = a.sum_out, p.ldsum = a.ldsum, p.w = a.w, p.y = a.y, p.ldy = a.ldy;
     p.dim = a.dim, p.eps = a.eps, p.normalize = a.normalize;
+    p.ssq = a.ssq, p.tiling = a.tiling;
     p.link = a.link;
     p.status = status_ptr();
     if (!p.status) return cudaErrorUnknown;
-    return launch_pdl(row_prep_kernel, dim3(a.rows), dim3(kRowThreads), 0, stream, p);
+    return launch_pdl(a.link.world > 0 ? row_prep_kernel<true> : row_prep_kernel<false>, dim3(a.rows), dim3(kRowThreads), 0, stream, p);
 }
 
 // ------------------------------------------------- QK-norm + RoPE + cache ---

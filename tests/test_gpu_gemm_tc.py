@@ -34,7 +34,7 @@ def test_batched_projection(B, N, K):
     assert torch.equal(first, Y)  # fixed order of the sums
 
 
-@pytest.mark.parametrize("B", [9, 32, 64])
+@pytest.mark.parametrize("B", [2, 8, 9, 32, 64])
 @pytest.mark.parametrize("H,I,NH", [(64, 16, 1), (1040, 1048 * 2, 3), (2048, 6144, 16)])
 def test_projection_epilogues(B, H, I, NH):
     """Residual and SwiGLU epilogues through the output projection + FFN operator, in 64 bits from the same rounding
