@@ -69,6 +69,7 @@ Trace trace_handle() { return g_trace; }
 
 static thread_local bool t_chain_first = false;
 void chain_begin() { t_chain_first = true; }
+bool chain_at_first() { return t_chain_first; }
 bool chain_take_first() {
     const bool f = t_chain_first;
     t_chain_first = false;
@@ -86,7 +87,7 @@ static const int kTuningDefaults[EZB_TUNE_COUNT] = {
     1,    // EZB_TUNE_GEMV_PREFETCH (one stage ahead of the dependency wait measured fastest in the chained layer)
     1,    // EZB_TUNE_GEMV_CTAS_PER_SM
     128,  // EZB_TUNE_ATTN_MIN_CHUNK
-    8,    // EZB_TUNE_ATTN_WAVES
+    0,    // EZB_TUNE_ATTN_WAVES (balanced schedule)
     0,    // EZB_TUNE_GEMV_KC (automatic)
     1,    // EZB_TUNE_GEMV_ROWS8
     0,    // EZB_TUNE_PDL_ACROSS_CALLS

@@ -474,6 +474,7 @@ unsigned int* status_ptr();   // device address of the status word on the curren
 Trace trace_handle();         // tracing buffers of the current device (buf == null when disabled)
 void chain_begin();           // marks the next launch_pdl() of this thread as the first kernel of a call
 bool chain_take_first();      // true once after chain_begin()
+bool chain_at_first();        // true until then
 void count_launch();          // one more kernel launch issued by the library (ezb_launch_count)
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -54,7 +54,7 @@ typedef struct CUstream_st* ezb_stream_t; /* same type as cudaStream_t */
 #define EZB_TUNE_GEMV_PREFETCH 2    /* weight stages requested before the dependency wait (0 = all; default 1) */
 #define EZB_TUNE_GEMV_CTAS_PER_SM 3 /* persistent CTAs per SM of the weight-streaming kernel            */
 #define EZB_TUNE_ATTN_MIN_CHUNK 4   /* smallest KV split, in keys (multiple of 64)                      */
-#define EZB_TUNE_ATTN_WAVES 5       /* target number of KV splits per SM                                */
+#define EZB_TUNE_ATTN_WAVES 5       /* rows of different lengths: 0 (default) = dealt out by their real lengths; n > 0 = n KV splits per SM on the grid of the longest row */
 #define EZB_TUNE_GEMV_KC 6          /* k-chunk length of a weight stage (0 = automatic)                 */
 #define EZB_TUNE_GEMV_ROWS8 7       /* 1: batch <= 8 uses the whole-row small-batch kernel (default 1)   */
 #define EZB_TUNE_PDL_ACROSS_CALLS 8 /* 1: the first kernel of a call may also start early (default 0)    */
