@@ -70,6 +70,7 @@ Trace trace_handle() { return g_trace; }
 static thread_local bool t_chain_first = false;
 void chain_begin() { t_chain_first = true; }
 bool chain_at_first() { return t_chain_first; }
+bool chain_waits_first() { return t_chain_first && !tuning(EZB_TUNE_PDL_ACROSS_CALLS); }
 bool chain_take_first() {
     const bool f = t_chain_first;
     t_chain_first = false;

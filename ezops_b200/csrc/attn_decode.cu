@@ -46,6 +46,7 @@ struct AttnParams {
     int B, H, NKV, S, G;
     int chunk, nchunks, nqt;
     int min_tiles;  // balanced schedule: smallest split, in tiles
+    int first;      // see pdl_open
     int early;      // the caches and lengths may be read before the dependency wait (see launch_attn_decode)
     float scale_log2e;
     float* part_o;   // [items][16][D]
@@ -166,7 +167,7 @@ __global__ void __launch_bounds__(kAttnThreads, D <= 64 ? 3 : 2) attn_decode_ker
     auto row_len = [&](int b) { return p.seq_lens ? max(p.fuse_new_token ? 1 : 0, min(p.S, p.seq_lens[b])) : p.S; };
 
     unsigned long long* trec = (tid == 0) ? trace_open(p.trace, 9u, cta) : nullptr;
-    pdl_trigger();
+    pdl_open(p.first);
     // This kernel is latency-bound at small batch; meanwhile HBM can already pull
     // the next kernel's weights (immutable, so safe before the dependency wait).
     if (warp == 3) prefetch_next_operands(p.next, lane, cta, gridDim.x * gridDim.y * gridDim.z);
@@ -840,6 +841,7 @@ cudaError_t launch_attn_decode(const AttnArgs& a, cudaStream_t stream) {
     p.min_tiles = max(1, tuning(EZB_TUNE_ATTN_MIN_CHUNK) / kTileKeys);
     // Inside a chain whose first kernel began after everything in front of it, the caches, the lengths and the page table
     // are complete before this kernel starts (not if calls may overlap).
+    p.first = chain_waits_first();
     p.early = tuning(EZB_TUNE_PDL) && !tuning(EZB_TUNE_PDL_ACROSS_CALLS) && !chain_at_first();
     p.fuse_new_token = a.fuse_new_token;
     p.qkv = a.qkv, p.qkv_bstride = a.qkv_bstride;

@@ -80,6 +80,7 @@ struct MegaParams {
                    // barrier behind gate/up
     unsigned int stage_bytes, act_bytes;
     long long wait_cycles;
+    int first;        // see pdl_open
     int evict_first;  // L2 evict-first policy on the streams: 1 = weights, 2 = weights and K/V
     unsigned int* status;
     Trace trace;
@@ -522,7 +523,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_layer_b1_kernel(const 
         mbar_fence_init();
     }
     __syncthreads();
-    pdl_trigger();
+    pdl_open(p.first);
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
@@ -1188,6 +1189,7 @@ cudaError_t launch_decode_mega(const MegaArgs& a, cudaStream_t stream) {
     p.NS = pl.NS;
     p.l2_window = tuning(EZB_TUNE_MEGA_L2_STAGES);
     if (p.l2_window < 0 || !tuning(EZB_TUNE_L2_PREFETCH)) p.l2_window = 0;
+    p.first = chain_waits_first();
     p.evict_first = tuning(EZB_TUNE_STREAM_EVICT_FIRST);
     p.inflight = tuning(EZB_TUNE_MEGA_INFLIGHT);
     if (p.inflight < 0 || p.inflight >= p.NS) p.inflight = 0;

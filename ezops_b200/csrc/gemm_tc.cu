@@ -49,6 +49,7 @@ struct TcParams {
     int log2c;            // log2 of the cluster size
     int cpc;              // batch columns that one CTA of the cluster finishes
     int nstages;
+    int first;            // see pdl_open
     int pair;             // 1: a tile holds `units` gate rows and `units` up rows, SwiGLU epilogue
     int epilogue;
     const bf16* residual;
@@ -267,7 +268,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     unsigned long long* trec = (tid == 64) ? trace_open(p.trace, (unsigned)p.trace_id, blockIdx.x) : nullptr;
-    pdl_trigger();
+    pdl_open(p.first);
     // The barriers above are initialised: peers may write here once they have passed the wait.  (A launch without a
     // cluster leaves the cluster barrier alone: there its wait held the epilogue until every warp of the CTA had come.)
     if (C > 1) cluster_arrive();
@@ -729,6 +730,7 @@ static cudaError_t launch_tc_instance(const GemvArgs& a, const bf16* x, long lon
     size_t smem = 0;
     if (!tc_plan<NB, LINK>(p, dev, clusters, smem)) return cudaErrorInvalidConfiguration;
     if (a.tiling && a.prologue != PRO_SCALED) a.tiling->units = p.units, a.tiling->tiles = p.tiles;
+    p.first = chain_waits_first();
     p.cols_pad = 1;
     while (p.cols_pad < p.cpc) p.cols_pad *= 2;
     alignas(64) CUtensorMap m0, m1, mx;

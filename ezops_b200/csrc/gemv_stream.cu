@@ -71,6 +71,7 @@ struct GemvParams {
     int nstages;   // ring depth
     int prefetch;  // stages requested before the dependency wait
     int window;    // at most this many stages requested but not yet landed (0 = no limit)
+    int first;        // see pdl_open
     int evict_first;  // 1: weight rows are read with the L2 evict-first policy
     unsigned int* status;
     PrefetchList next;
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_stream_kernel(const Gemv
         mbar_fence_init();
     }
     __syncthreads();
-    pdl_trigger();
+    pdl_open(p.first);
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
@@ -564,7 +565,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows8_kernel(const GemvP
     }
     unsigned long long* trec = (tid == 32) ? trace_open(p.trace, (unsigned)p.trace_id, blockIdx.x) : nullptr;
     __syncthreads();
-    pdl_trigger();
+    pdl_open(p.first);
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
@@ -949,6 +950,7 @@ cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream) {
         p.prologue = tc_args.prologue = defer ? PRO_SCALED : PRO_NONE;
         if (defer && !a.norm_w) p.x = a.x_sum_out, p.ldx = a.ldsum;
     }
+    p.first = chain_waits_first();
     if (use_tc) return launch_gemm_tc(tc_args, p.x, p.ldx, stream);
 
     if (rows8) {

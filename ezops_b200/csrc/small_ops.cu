@@ -30,8 +30,7 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_f32_kernel(const float* _
                                                                   int dim, float eps, int staged) {
     extern __shared__ __align__(16) float row_s[];
     __shared__ float scratch[8];
-    pdl_trigger();
-    pdl_wait();
+    pdl_open(1);
     const float* x = X + (long long)blockIdx.x * dim;
     float* o = Out + (long long)blockIdx.x * dim;
     const bool vec = (dim & 3) == 0;
@@ -83,6 +82,7 @@ struct RowPrepParams {
     int dim;
     float eps;
     int normalize;
+    int first;  // see pdl_open
     float* ssq;
     TcTiling tiling;
     TpLink link;
@@ -120,8 +120,7 @@ __device__ __forceinline__ uint4 load_row8(const RowPrepParams& p, long long row
 // a graph of {copy in, layer, copy out} needs no hand-over between the copy engines and the SMs.
 __global__ void __launch_bounds__(256) pinned_copy_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, long long n16,
                                                           int to_host) {
-    pdl_trigger();
-    pdl_wait();  // src may be what the kernel in front wrote; dst may be what it still reads
+    pdl_open(1);  // src may be what the kernel in front wrote; dst may be what it still reads
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += (long long)gridDim.x * blockDim.x) dst[i] = src[i];
     if (to_host) __threadfence_system();
 }
@@ -138,7 +137,7 @@ cudaError_t launch_pinned_copy(void* dst, const void* src, size_t bytes, bool to
 template <bool LINK>
 __global__ void __launch_bounds__(kRowThreads) row_prep_kernel(const RowPrepParams p) {
     __shared__ float scratch[8];
-    pdl_trigger();
+    pdl_open(p.first);
     pdl_wait();
     const bool gather = LINK && p.link.world > 0 && p.link.gather_inbox >= 0;
     if (gather && tp_poisoned(p.status)) return;  // see tp_poisoned: the chain already gave up a wait
@@ -221,6 +220,7 @@ cudaError_t launch_row_prep(const RowPrepArgs& a, cudaStream_t stream) {
     p.x = a.x, p.ldx = a.ldx, p.add = a.add, p.ldadd = a.ldadd;
     p.sum_out = a.sum_out, p.ldsum = a.ldsum, p.w = a.w, p.y = a.y, p.ldy = a.ldy;
     p.dim = a.dim, p.eps = a.eps, p.normalize = a.normalize;
+    p.first = chain_waits_first();
     p.ssq = a.ssq, p.tiling = a.tiling;
     p.link = a.link;
     p.status = status_ptr();
@@ -246,8 +246,7 @@ struct RopeParams {
 static constexpr int kRopeMaxPairsPerLane = 8;  // D <= 512
 
 __global__ void __launch_bounds__(128) qk_norm_rope_kernel(const RopeParams p) {
-    pdl_trigger();
-    pdl_wait();
+    pdl_open(1);
     const int lane = threadIdx.x & 31;
     const int unit = blockIdx.x * 4 + (threadIdx.x >> 5);
     const int heads = p.NQ + p.NKV;

@@ -15,10 +15,12 @@
  *   - Work is enqueued on `stream` and the call returns without synchronising,
  *     so calls can be captured into a CUDA graph.  The kernels of one call are
  *     chained with programmatic dependent launch: a kernel may start while its
- *     predecessor drains and request WEIGHT tiles early, but reads activations
- *     and the KV cache only after the predecessor has finished.  The first kernel
- *     of a call is ordered against earlier work on the stream in the usual way,
- *     unless EZB_TUNE_PDL_ACROSS_CALLS is set; set it only when the weight
+ *     predecessor drains and request WEIGHT tiles, norm weights, rotary rows and
+ *     cached keys and values early, but reads activations only after the
+ *     predecessor has finished.  The first kernel of a call may be resident early
+ *     too, but it and everything behind it touch nothing before all earlier work
+ *     on the stream has finished, unless EZB_TUNE_PDL_ACROSS_CALLS is set (cached
+ *     keys and values are then not read early); set it only when the weight
  *     tensors are not written by work enqueued shortly before the call (a decode
  *     loop over resident weights), since early weight requests then overlap the
  *     tail of the previous call.
