@@ -46,7 +46,7 @@ namespace ezb {
 static constexpr int kMegaConsumerWarps = 8;
 static constexpr int kMegaConsumerThreads = kMegaConsumerWarps * 32;
 static constexpr int kMegaThreads = 32 + kMegaConsumerThreads;
-static constexpr int kMegaMaxStages = 8;
+static constexpr int kMegaMaxStages = 12;
 static constexpr int kMegaHeaderBytes = 512;   // barriers, abort flag, norm scratch, flags
 static constexpr int kMegaRedGroup = 4;        // row blocks whose partial sums are combined across the warps in one go
 static constexpr int kMegaRedBytes = 2 * kMegaRedGroup * kMegaConsumerWarps * 8 * (int)sizeof(float);
@@ -1115,7 +1115,12 @@ static bool mega_plan(const MegaArgs& a, MegaPlan& pl) {
     const int grid = sm_count();
     if (a.NKV > grid) return false;
     if ((a.H + grid - 1) / grid + 1 > kMegaResSlots) return false;
-    auto kc_of = [](int K) { return K < 4096 ? K : 4096; };
+    // A stage is sized for the longest row piece but holds eight rows of every phase: with pieces of 4096 a model of 2048
+    // hidden units fills half of its 64 KB stages, and the ring of three holds 96 KB.  Pieces of its own row length keep
+    // the ring full of useful bytes (2B layer, KV 1024: 40.5 -> 38.2 us).  Shorter rows keep the longer pieces of the
+    // other phases: cutting those to 1024 made the 0.6B layer 1..3 us slower (27.4 -> 28.4, KV 4096 30.2 -> 33.2).
+    const int cap_kc = (a.H > 1024 && a.H <= 2048) ? 2048 : 4096;
+    auto kc_of = [cap_kc](int K) { return K < cap_kc ? K : cap_kc; };
     pl.grid = grid;
     pl.kc_h = kc_of(a.H), pl.kc_q = kc_of(Q), pl.kc_i = kc_of(a.I);
     const int kc_max = pl.kc_h > pl.kc_q ? (pl.kc_h > pl.kc_i ? pl.kc_h : pl.kc_i) : (pl.kc_q > pl.kc_i ? pl.kc_q : pl.kc_i);
@@ -1191,7 +1196,8 @@ cudaError_t launch_decode_mega(const MegaArgs& a, cudaStream_t stream) {
     if (p.l2_window < 0 || !tuning(EZB_TUNE_L2_PREFETCH)) p.l2_window = 0;
     p.first = chain_waits_first();
     p.evict_first = tuning(EZB_TUNE_STREAM_EVICT_FIRST);
-    p.inflight = tuning(EZB_TUNE_MEGA_INFLIGHT);
+    // the tuning value counts stages of 64 KB
+    p.inflight = (int)((size_t)tuning(EZB_TUNE_MEGA_INFLIGHT) * 8 * (4096 + kMegaRowPad) * 2 / pl.stage_bytes);
     if (p.inflight < 0 || p.inflight >= p.NS) p.inflight = 0;
     p.gate = tuning(EZB_TUNE_MEGA_GATE) & 7;
     p.stage_bytes = (unsigned int)pl.stage_bytes, p.act_bytes = (unsigned int)pl.act_bytes;

@@ -72,7 +72,7 @@ typedef struct CUstream_st* ezb_stream_t; /* same type as cudaStream_t */
 #define EZB_TUNE_MEGA_L2_STAGES 18    /* single-kernel layer: stages a producer with a full ring may pull into L2 ahead (default 0) */
 #define EZB_TUNE_WAIT_LIMIT_MS 19     /* budget of one device-side wait in the single-kernel layer and the cross-rank waits, ms at 2 GHz (default 1000) */
 #define EZB_TUNE_MEGA_STAGES 20       /* single-kernel layer: cap on the ring depth (0 = as many as fit)                            */
-#define EZB_TUNE_MEGA_INFLIGHT 21     /* single-kernel layer: stages that may be requested but not yet landed (0 = whole ring; default 2) */
+#define EZB_TUNE_MEGA_INFLIGHT 21     /* single-kernel layer: what may be requested but not yet landed, in stages of 64 KB (0 = whole ring; default 2) */
 #define EZB_TUNE_MEGA_GATE 22         /* single-kernel layer, bit mask: a producer stops 1 = behind its K/V stages until the QKV barrier is passed (default), 2 = behind Wo until the barrier after o_proj, 4 = behind gate/up until the barrier after it */
 #define EZB_TUNE_TP_WAIT_LIMIT_MS 23   /* fused exchange: budget of one wait for the peers' partial sums, ms at 2 GHz (default 5000)      */
 #define EZB_TUNE_TP_STRONG_STORES 24   /* fused exchange: 1 = publish cells with st.relaxed.sys instead of plain stores (default 0) */
