@@ -296,9 +296,9 @@ def roofline_leg(sets, nsets, hidden0, B, H, device, n_roof):
     launch_s = r0.elapsed_time(r1) * 1e-3 / n_roof
     kernel_bytes = 2 * (rows_local * H + B * H + B * rows_local)
     achieved = kernel_bytes / launch_s / 1e9
-    traffic, traffic_how = ncu_traffic("gemv_rows8_kernel" if B <= 8 else "gemm_tc_kernel", rows_local, H, B)
+    traffic, traffic_how = ncu_traffic("gemv_rows8_kernel" if B == 1 else "gemm_tc_kernel", rows_local, H, B)
     roofline = {
-        "bound": "hbm", "kernel": "gemv_rows8_kernel" if B <= 8 else "gemm_tc_kernel", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
+        "bound": "hbm", "kernel": "gemv_rows8_kernel" if B == 1 else "gemm_tc_kernel", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
         "frac": achieved / peaks["hbm_gbs"], "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs, burst copy)",
         "traffic": traffic, "traffic_source": traffic_how, "bytes_per_launch": kernel_bytes, "us_per_launch": launch_s * 1e6,
         "workload": f"W [{rows_local}, {H}] bf16 (gate/up-sized), batch {B}, {n_roof} back-to-back launches over {nsets} weights",
