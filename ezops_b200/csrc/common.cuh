@@ -262,20 +262,20 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Wait for the phase with the given parity, for at most kWaitLimitCycles.
+// Wait for the phase with the given parity, for at most `limit` cycles.
 // `abort_flag` lives in shared memory: once any thread of the CTA has given
 // up, every later wait in the CTA returns at once, so the control flow of all
 // warps (and the named barriers they meet at) stays the same and the CTA runs
 // to its end without hanging.  Returns false when it gave up.
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                                  unsigned int* status, unsigned int fault_code) {
+                                                  unsigned int* status, unsigned int fault_code, long long limit = kWaitLimitCycles) {
     if (mbar_try_wait(bar, parity)) return true;
     if (*abort_flag) return false;
     const long long t0 = clock64();
     for (;;) {
         if (mbar_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
-        if (clock64() - t0 > kWaitLimitCycles) {
+        if (clock64() - t0 > limit) {
             *abort_flag = 1;
             report_fault(status, fault_code);
             return false;

@@ -1201,7 +1201,8 @@ cudaError_t launch_decode_mega(const MegaArgs& a, cudaStream_t stream) {
     if (p.inflight < 0 || p.inflight >= p.NS) p.inflight = 0;
     p.gate = tuning(EZB_TUNE_MEGA_GATE) & 7;
     p.stage_bytes = (unsigned int)pl.stage_bytes, p.act_bytes = (unsigned int)pl.act_bytes;
-    p.wait_cycles = wait_limit_cycles();
+    // A wait behind an exchange (a full ring, the next grid barrier) lasts as long as another CTA's wait for the peers.
+    p.wait_cycles = wait_limit_cycles() + (a.link.world > 0 ? a.link.wait_cycles : 0);
     p.status = status_ptr();
     if (!p.status) return cudaErrorUnknown;
     p.trace = trace_handle();

@@ -329,6 +329,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant_
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         if (elect_one()) {
+            // A stage is full only with the X block that the producer requests behind its own dependency wait.  Waiting
+            // here too keeps the time that the kernel in front takes - a gather may wait for its peers for seconds, and
+            // has released this kernel before - out of the budget of the waits below.
+            pdl_wait();
             int stage = 0;
             uint32_t full_parity = 0;
             for (int i = 0; i < my_tiles && !(*abort_flag); ++i) {

@@ -604,11 +604,13 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows8_kernel(const GemvP
             if (ok) request(it);
         }
         pdl_wait();
+        // the consumers may first wait for the peers, and hand back no stage until then
+        const long long limit = kWaitLimitCycles + (LINK && p.link.world > 0 && p.link.gather_inbox >= 0 ? p.link.wait_cycles : 0);
         int issued = ok ? npre : 0;
         for (int it = npre; it < total && ok; ++it) {
             const int s = it % NS;
             const uint32_t parity = (uint32_t)(((it / NS) & 1) ^ 1);
-            if (!mbar_wait_bounded(smem_u32(&empty_bar[s]), parity, abort_flag, p.status, FAULT_GEMV_EMPTY_WAIT)) break;
+            if (!mbar_wait_bounded(smem_u32(&empty_bar[s]), parity, abort_flag, p.status, FAULT_GEMV_EMPTY_WAIT, limit)) break;
             if (W > 0 && it >= W && !landed(it - W)) break;
             request(it);
             issued = it + 1;

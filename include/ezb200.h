@@ -70,7 +70,7 @@ typedef struct CUstream_st* ezb_stream_t; /* same type as cudaStream_t */
 #define EZB_TUNE_TP_PULL 16           /* fused exchange direction: 0 = push (default), 1 = pull (consumers read the peers' buffers) */
 #define EZB_TUNE_MEGA 17              /* 1: the batch-1 decode layer runs as one persistent kernel when the shape allows (default 1) */
 #define EZB_TUNE_MEGA_L2_STAGES 18    /* single-kernel layer: stages a producer with a full ring may pull into L2 ahead (default 0) */
-#define EZB_TUNE_WAIT_LIMIT_MS 19     /* budget of one device-side wait in the single-kernel layer and the cross-rank waits, ms at 2 GHz (default 1000) */
+#define EZB_TUNE_WAIT_LIMIT_MS 19     /* budget of one device-side wait in the single-kernel layer, ms at 2 GHz (default 1000; with the fused exchange plus the limit below) */
 #define EZB_TUNE_MEGA_STAGES 20       /* single-kernel layer: cap on the ring depth (0 = as many as fit)                            */
 #define EZB_TUNE_MEGA_INFLIGHT 21     /* single-kernel layer: what may be requested but not yet landed, in stages of 64 KB (0 = whole ring; default 2) */
 #define EZB_TUNE_MEGA_GATE 22         /* single-kernel layer, bit mask: a producer stops 1 = behind its K/V stages until the QKV barrier is passed (default), 2 = behind Wo until the barrier after o_proj, 4 = behind gate/up until the barrier after it */
