@@ -164,7 +164,9 @@ __global__ void __launch_bounds__(kAttnThreads, D <= 64 ? 3 : 2) attn_decode_ker
     const int g4 = lane >> 2, t4 = lane & 3;
     const int G = p.G;
     const int cta = SCHED ? (int)blockIdx.x : (int)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
-    auto row_len = [&](int b) { return p.seq_lens ? max(p.fuse_new_token ? 1 : 0, min(p.S, p.seq_lens[b])) : p.S; };
+    // Lengths and page ids may be read before the dependency wait (`early`): through L2, since a line that an earlier
+    // kernel left in this SM's L1 is only known to be dropped behind that wait.
+    auto row_len = [&](int b) { return p.seq_lens ? max(p.fuse_new_token ? 1 : 0, min(p.S, __ldcg(p.seq_lens + b))) : p.S; };
 
     unsigned long long* trec = (tid == 0) ? trace_open(p.trace, 9u, cta) : nullptr;
     pdl_open(p.first);
@@ -302,7 +304,7 @@ __global__ void __launch_bounds__(kAttnThreads, D <= 64 ? 3 : 2) attn_decode_ker
     auto cache_row = [&](const AttnSegment& sg, int key, bool& ok) -> long long {
         ok = true;
         if (!p.page_table) return ((long long)sg.b * p.NKV + sg.kvh) * p.S + key;
-        const long long page = __ldg(p.page_table + (long long)sg.b * p.max_pages + (key >> p.page_shift));
+        const long long page = __ldcg(p.page_table + (long long)sg.b * p.max_pages + (key >> p.page_shift));
         if (page < 0 || page >= p.num_pages) {
             report_fault(p.status, FAULT_PAGE_RANGE);
             ok = false;
