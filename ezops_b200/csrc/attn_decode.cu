@@ -811,7 +811,18 @@ static cudaError_t launch_attn_instance(AttnParams& p, void* records, cudaStream
         // 128..1024 keys, 28 layers: 858 us, 886 with the schedule computed in front of every layer's attention).
         const int cut = min(p.min_tiles * kTileKeys, (p.S + kTileKeys - 1) / kTileKeys * kTileKeys);
         const int n = (p.S + cut - 1) / cut;
-        if ((long long)p.B * p.NKV * p.nqt * n <= slots) sched = false, p.chunk = cut, p.nchunks = n;
+        const long long groups = (long long)p.B * p.NKV * p.nqt;
+        if (groups * n <= slots) sched = false, p.chunk = cut, p.nchunks = n;
+        // Where the fixed grid does not cut a row either (a row is one split, or there are so many that each gets a CTA
+        // of its own) the hardware hands out the groups one by one, which beats fixed shares of them: 64 rows of 13..100
+        // keys 8.4 us on the grid, 15.5 by schedule; 128 rows of 48..384 keys 28 and 40; 45 rows of 112..900 keys and 32
+        // kv heads 58 and 68; even from about 3000 keys on.
+        else if (p.nchunks == 1) sched = false;
+        // Head dim 64: a new group costs as much as at 128 but its tiles cost half, so the schedule gains only where groups
+        // are few and long (11 rows of 512..4096 keys 17.3 us on the grid, 14.8 by schedule) and loses elsewhere (64 rows of
+        // 64..512 keys 15.2 and 19.5).  Over 2000 shapes this rule is 11..14 % faster than the schedule wherever something
+        // is cut, the grid everywhere 10..12 %.
+        else if (D <= 64 && (2 * groups > slots || tiles <= 4LL * slots)) sched = false;
     }
     const size_t items = sched ? 2 * (size_t)slots : (size_t)p.B * p.NKV * p.nqt * p.nchunks;
     p.part_ml = static_cast<float*>(records);

@@ -15,10 +15,12 @@ CASES = [
     (1, 8, 8, 200, 64, 1),  # one row, a few tiles
     (4, 16, 8, 640, 128, 0),  # empty rows among them
     (13, 16, 8, 1024, 128, 128),  # pieces
-    (64, 32, 8, 100, 128, 1),  # whole groups
+    (64, 32, 8, 100, 128, 1),  # one CTA per group
     (64, 16, 8, 300, 64, 0),
+    (96, 32, 8, 300, 128, 1),  # whole groups
     (24, 32, 8, 3000, 128, 100),  # ranges
-    (40, 8, 8, 4096, 64, 1),  # ranges, head_dim 64
+    (24, 8, 8, 4096, 64, 1),  # ranges, head_dim 64
+    (40, 8, 8, 4096, 64, 1),  # fixed grid, head_dim 64
     (128, 16, 8, 257, 128, 1),  # the most rows the schedule covers
     (129, 8, 8, 257, 128, 1),  # one more
     (2, 64, 2, 3000, 128, 10),  # two query tiles per kv head
@@ -57,3 +59,35 @@ def test_ragged_attention(B, H, NKV, S, D, low):
         q, k, v = Q[b, :, 0].double().view(NKV, H // NKV, D), K[b, :, :n].double(), V[b, :, :n].double()
         want = ((q @ k.transpose(1, 2) * D**-0.5).softmax(-1) @ v).reshape(H, D)
         assert ((outs[0][b, :, 0].double() - want).norm() / want.norm()).item() < 6e-3, (b, n)
+
+
+@pytest.mark.parametrize("B,H,NKV,S,D,ctas", [
+    (64, 32, 8, 100, 128, 64 * 8),  # a row is one split: one CTA per (row, kv head)
+    (128, 32, 8, 384, 128, 128 * 8),  # more groups than the fixed grid cuts
+    (64, 32, 8, 512, 64, 64 * 8 * 2),  # head_dim 64, many short groups: two splits each
+    (4, 16, 8, 1024, 128, 4 * 8 * 8),  # the smallest splits of full rows fit one wave
+    (32, 32, 8, 8192, 128, None),  # balanced: two CTAs per SM
+    (11, 32, 8, 4096, 64, None),  # head_dim 64, few long groups: three
+])
+def test_which_shapes_are_balanced(B, H, NKV, S, D, ctas):
+    """Which grid a batch of rows of different lengths runs on (trace records: one per CTA).  The balanced schedule is slower
+    where the hardware hands out whole groups one by one, see launch_attn_instance."""
+    if ctas is None:
+        ctas = torch.cuda.get_device_properties(0).multi_processor_count * (2 if D == 128 else 3)
+    rng = random.Random(B)
+    lens = torch.tensor([rng.randint(S // 8, S) for _ in range(B)], dtype=torch.int32, device="cuda")
+    Q, out = (torch.zeros(B, H, 1, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    K, V = (torch.zeros(B, NKV, S, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    lib = _lib.load()
+    ws = torch.zeros(lib.ezb_attn_decode_workspace_bytes(B, H, NKV, S, D), dtype=torch.uint8, device="cuda")
+    records = torch.zeros(4096 * 6, dtype=torch.int64, device="cuda")
+    cursor = torch.zeros(1, dtype=torch.int32, device="cuda")
+    try:
+        _lib.check(lib.ezb_trace_enable(records.data_ptr(), cursor.data_ptr(), 4096))
+        _lib.check(lib.ezb_attn_decode(Q.data_ptr(), K.data_ptr(), V.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel(), B, H, NKV, S, D,
+                                       lens.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+    finally:
+        _lib.check(lib.ezb_trace_enable(None, None, 0))
+    assert cursor.item() == ctas
+    assert _lib.device_status() == 0
