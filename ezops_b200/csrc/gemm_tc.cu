@@ -707,7 +707,11 @@ static bool tc_plan(TcParams& p, int dev, int& clusters, size_t& smem) {
             if (half && !all) continue;  // a long stream wants the deeper ring
             const double block = 40. + 2.6 * (p.pair ? 2 * units : units) + 0.9 * NB;
             const double tile = nk * (block < 150. ? 150. : block), epi = (C > 1 ? 1100. : 800.) + 60. * cpc;
-            const double cost = rounds * tile + (rounds - 1) * (epi > tile ? epi - tile : 0.) + epi;
+            // The next tile's MMAs hide this one's epilogue, but an exchange keeps its buffers until every CTA of the cluster
+            // has read them: 4 us from the last MMA on, whatever the batch.  Shorter tiles wait for it (N = 151936, K =
+            // 1024, batch 16 | 32 | 64: 53 | 57 | 60 us on one CTA per tile, 66 | 72 | 74 on two, 95 | 105 | 122 on four).
+            const double hidden = C > 1 && epi < 4000. ? 4000. : epi;
+            const double cost = rounds * tile + (rounds - 1) * (hidden > tile ? hidden - tile : 0.) + epi;
             if (best > 0. && cost >= best) continue;
             best = cost;
             p.log2c = log2c, p.cpc = cpc, p.units = units, p.half_rows = half_rows, p.a_rows = a_rows, p.tiles = tiles;
