@@ -422,7 +422,13 @@ int ezb_gemv_batched_bf16(const void* X, const void* W, void* Y, void* workspace
     g.W0 = static_cast<const bf16*>(W), g.ldw = K, g.N = N, g.K = K, g.B = B;
     g.x = static_cast<const bf16*>(X), g.ldx = K;
     g.out = Y, g.ldout = N;
-    g.allow_tc = B >= 2;
+    // Up to four rows and few outputs: the whole weight is on its way before the rows are staged, and the small-batch kernel
+    // ends sooner than the exchange between CTAs that the tensor-core kernel needs there (weights from HBM, 2 rows, us: N =
+    // 1024, K = 8192 6.4 | 7.9; 2048 x 3072 5.7 | 6.9; above 2048 outputs it depends on how the rows divide: 3072 x 4096
+    // 8.6 | 9.1, 4096 x 4096 10.3 | 9.3, 6144 x 3072 11.6 | 10.7).  Inside a layer the tensor-core kernel is the faster
+    // one: it takes over the norms (see gemv_uses_tc).
+    const bool small = B <= 4 && (long long)B * K <= 16384 && N <= 2048 && gemv_small_batch_eligible(B, K);
+    g.allow_tc = B >= 2 && !small;
     chain_begin();
     EZB_CUDA_TRY(launch_gemv(g, stream));
     return EZB_OK;

@@ -54,3 +54,33 @@ def test_projection_epilogues(B, H, I, NH):
     want = x2 + (torch.nn.functional.silu(xn @ Wg.double().T) * (xn @ Wu.double().T)) @ Wd.double().T
     assert ((out.double() - want).norm() / want.norm()).item() < 1e-2
     assert torch.equal(out, op(attn, residual, Wo, w, Wg, Wu, Wd))
+
+
+@pytest.mark.parametrize("B,N,K,small", [
+    (2, 2048, 8192, True),  # rows x K up to 16384, 2048 outputs
+    (4, 2048, 4096, True),
+    (3, 130, 1024, True),
+    (4, 2048, 4128, False),  # past each edge
+    (2, 2049, 1024, False),
+    (5, 1024, 1024, False),
+    (2, 1024, 80, False),  # K the small-batch kernel does not take
+])
+def test_which_kernel_a_small_batch_runs_on(B, N, K, small):
+    """Both sides of the rule of ezb_gemv_batched_bf16: right values on each, and inside it the bits of the small-batch
+    kernel (the tensor cores add in another order, which shows in a few of so many roundings)."""
+    test_batched_projection(B, N, K)
+    if not small:
+        return
+    lib = _lib.load()
+    X, W = (torch.randn(n, K, device="cuda").bfloat16() for n in (B, N))
+    ws = torch.zeros(lib.ezb_gemv_workspace_bytes(B, N, K), dtype=torch.uint8, device="cuda")
+    got = []
+    try:
+        for tc in (1, 0):
+            _lib.set_tuning(tc=tc)
+            got.append(torch.empty(B, N, device="cuda", dtype=torch.bfloat16))
+            _lib.check(lib.ezb_gemv_batched_bf16(X.data_ptr(), W.data_ptr(), got[-1].data_ptr(), ws.data_ptr(), ws.numel(), B, N, K,
+                                                 torch.cuda.current_stream().cuda_stream))
+    finally:
+        _lib.set_tuning(tc=1)
+    assert torch.equal(*got)
