@@ -10,7 +10,7 @@ from ezops_b200 import _lib
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("B", [9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("B", [2, 3, 5, 8, 9, 16, 17, 32, 33, 64])
 @pytest.mark.parametrize("N,K", [(1, 16), (8, 64), (9, 80), (130, 80), (1024, 2048), (1023, 4112), (4097, 64), (10240, 144), (40001, 256)])
 def test_batched_projection(B, N, K):
     """Against the fp32 product: bf16 products are exact in fp32, so what differs is the order of K fp32 additions
@@ -54,6 +54,83 @@ def test_projection_epilogues(B, H, I, NH):
     want = x2 + (torch.nn.functional.silu(xn @ Wg.double().T) * (xn @ Wu.double().T)) @ Wd.double().T
     assert ((out.double() - want).norm() / want.norm()).item() < 1e-2
     assert torch.equal(out, op(attn, residual, Wo, w, Wg, Wu, Wd))
+
+
+# ------------------------------------------------------------------------------------ epilogues, value by value ---
+STEP = 2.0**-8  # a rounding to bf16 changes a value by at most this share of it; 2**-8.8 is its standard deviation at most
+BATCHES = [2, 3, 5, 8, 9, 17, 32, 64]
+SIZES = [(64, 16, 1), (1040, 2096, 3), (2048, 6144, 16)]  # H, I, heads of 64
+
+
+def _ffn(B, H, I, NH, seed):
+    import ezops_b200 as ez
+
+    g = torch.Generator().manual_seed(seed)
+    rand = lambda *s, std=1.0, mean=0.0: (torch.randn(*s, generator=g) * std + mean).bfloat16().cuda()  # noqa: E731
+    return ez.FusedOProjFfnOp(B, H, I, NH, 64, backend="cuda"), rand
+
+
+@pytest.mark.parametrize("B", BATCHES)
+@pytest.mark.parametrize("H,I,NH", SIZES)
+def test_residual_epilogue_value_by_value(B, H, I, NH):
+    """The FFN's last projection is zero, so the operator returns residual + attn Wo^T: every value of it within the
+    rounding of the product, that of the sum, and Q fp32 additions (at most 2**-24 of the magnitudes each)."""
+    op, rand = _ffn(B, H, I, NH, B + H)
+    Q = NH * 64
+    attn, residual, Wo, w = rand(B, Q), rand(B, H, std=0.5), rand(H, Q, std=Q**-0.5), rand(H, std=0.1, mean=1.0)
+    Wg, Wu, Wd = rand(I, H, std=0.02), rand(I, H, std=0.02), torch.zeros(H, I, device="cuda", dtype=torch.bfloat16)
+    out = op(attn, residual, Wo, w, Wg, Wu, Wd)
+    assert _lib.device_status() == 0
+    prod = attn.double() @ Wo.double().T
+    want = residual.double() + prod
+    bound = STEP * (prod.abs() + want.abs()) + Q * 2.0**-24 * (attn.double().abs() @ Wo.double().abs().T)
+    assert ((out.double() - want).abs() <= 1.01 * bound).all()
+
+
+@pytest.mark.parametrize("B", BATCHES)
+@pytest.mark.parametrize("H,I,NH", SIZES)
+def test_swiglu_and_deferred_norm_value_by_value(B, H, I, NH):
+    """The output projection is zero and the last projection picks one value of silu(gate) * up per output, so the
+    operator returns residual + that value; shifted picks return every one of them.  gate and up are sums of products of
+    rows rounded to bf16 once: independent errors, within eight standard deviations; then one rounding each, and one
+    each for silu, the product and the sum.  silu has slope 1.1 at most."""
+    op, rand = _ffn(B, H, I, NH, 7 * B + H)
+    Q = NH * 64
+    attn, residual, w = rand(B, Q), rand(B, H, std=0.0625), rand(H, std=0.1, mean=1.0)
+    Wo = torch.zeros(H, Q, device="cuda", dtype=torch.bfloat16)
+    Wg, Wu = rand(I, H, std=H**-0.5), rand(I, H, std=H**-0.5)
+    x = residual.double()
+    xn = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+
+    def project(W):
+        v = xn @ W.double().T
+        return v, STEP * v.abs() + 8 * 2.0**-8.8 * (xn.square() @ W.double().square().T).sqrt()
+
+    (gate, dg), (up, du) = project(Wg), project(Wu)
+    s = torch.nn.functional.silu(gate)
+    h = s * up
+    ds = 1.1 * dg + STEP * s.abs()
+    dh = (up.abs() + du) * ds + (s.abs() + ds) * du + STEP * h.abs()
+    j = torch.arange(H, device="cuda")
+    for first in range(0, I, H):
+        pick = (j + first) % I
+        Wd = torch.zeros(H, I, device="cuda", dtype=torch.bfloat16)
+        Wd[j, pick] = 1.0
+        out = op(attn, residual, Wo, w, Wg, Wu, Wd)
+        want = x + h[:, pick]
+        assert ((out.double() - want).abs() <= 1.01 * (dh[:, pick] + STEP * (want.abs() + dh[:, pick]))).all()
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("B", [2, 5, 8])
+@pytest.mark.parametrize("N,K", [(1, 32), (8, 64), (130, 96), (1023, 4128), (4097, 64), (2048, 4096)])
+def test_small_batch_kernel_without_the_tensor_cores(B, N, K):
+    """What EZB_TUNE_TC = 0 selects for 2 to 8 rows (csrc/gemv_stream.cu); the bound of test_batched_projection."""
+    try:
+        _lib.set_tuning(tc=0)
+        test_batched_projection(B, N, K)
+    finally:
+        _lib.set_tuning(tc=1)
 
 
 @pytest.mark.parametrize("B,N,K,small", [
