@@ -34,6 +34,8 @@ static constexpr int kAttnThreads = 128;
 static constexpr int kTileKeys = 64;
 static constexpr int kAttnStages = 3;
 static constexpr int kSchedRows = 128;  // batch rows that the balanced schedule covers
+// CTAs of the kernel that share an SM: bounded by registers at head_dim 64 (160 a thread), by shared memory at 128.
+__host__ __device__ constexpr int attn_ctas_per_sm(int D) { return D <= 64 ? 3 : 2; }
 
 struct AttnParams {
     const bf16* Q;
@@ -145,7 +147,7 @@ struct AttnSchedule {
 };
 
 template <int D, bool SCHED>
-__global__ void __launch_bounds__(kAttnThreads, D <= 64 ? 3 : 2) attn_decode_kernel(const AttnParams p) {
+__global__ void __launch_bounds__(kAttnThreads, attn_ctas_per_sm(D)) attn_decode_kernel(const AttnParams p) {
     constexpr int CPR = D / 8;                       // 16-byte chunks per key row
     constexpr int ROW_BYTES = D * 2;
     constexpr int TILE_BYTES = kTileKeys * ROW_BYTES;  // one K or V tile
@@ -725,15 +727,17 @@ __global__ void __launch_bounds__(kAttnThreads, D <= 64 ? 3 : 2) attn_decode_ker
 // head) as the resident slots allow, never more.  A second, partly filled wave costs a whole extra pass over a split
 // (Qwen3-8B layer, KV 4096, batch 2 / 4 / 8 / 16 / 32: 94.5 / 110.5 / 126.8 / 147.1 / 191.4 us with splits sized for
 // 1.5 waves, 89.5 / 107.4 / 124.6 / 141.2 / 181.6 with this rule; a sweep over every split length confirmed the
-// optimum at ~256 CTAs for each).  Ragged batches get the balanced schedule (AttnSchedule); with more rows than that
-// covers, or EZB_TUNE_ATTN_WAVES > 0, they are cut into more, shorter splits, because every row is then cut on the grid
-// of the longest row and short splits balance better.
+// optimum at ~256 CTAs for each).  Head dim 64 (32 heads over 8 kv heads; splits for four CTAs per SM, of which three are
+// resident | this rule): 1 row of 8192 keys 13.5 | 10.3 us, 8 rows of 4096 16.2 | 13.4, 24 rows of 2048 21.8 | 18.6.
+// Ragged batches get the balanced schedule (AttnSchedule) where launch_attn_instance says so.  Elsewhere, with more rows
+// than it covers, or with EZB_TUNE_ATTN_WAVES > 0, they are cut into more, shorter splits, because every row is then cut on
+// the grid of the longest row and short splits balance better.
 int attn_chunk_keys(int B, int NKV, int S, bool ragged, int D) {
     const long long total = (long long)B * NKV * S;
     const int waves = tuning(ragged ? EZB_TUNE_ATTN_WAVES : EZB_TUNE_ATTN_WAVES_UNIFORM);
     long long chunk;
     if (!ragged && waves <= 0) {
-        const long long slots = (long long)sm_count() * (D <= 64 ? 4 : 2);  // resident CTAs: the ring is 3 x 2 x 64 keys x D
+        const long long slots = (long long)sm_count() * attn_ctas_per_sm(D);
         long long splits = slots / ((long long)B * NKV);
         if (splits < 1) splits = 1;
         chunk = (S + splits - 1) / splits;
@@ -782,7 +786,6 @@ static int attn_slots() {
     if (keep) cache[dev].store(n, std::memory_order_relaxed);
     return n;
 }
-static constexpr int kSlotsPerSmMax = 4;  // what the workspace is sized for
 
 size_t attn_workspace_bytes(int B, int H, int NKV, int S, int D) {
     const int G = H / NKV, nqt = (G + 15) / 16;
@@ -791,7 +794,7 @@ size_t attn_workspace_bytes(int B, int H, int NKV, int S, int D) {
     size_t items = (size_t)B * NKV * nqt * nchunks;
     // the balanced schedule keeps two records per CTA of its grid, which never exceeds the number of tiles
     const size_t tiles = (size_t)B * NKV * nqt * ((S + kTileKeys - 1) / kTileKeys);
-    size_t slots = (size_t)sm_count() * (D <= 64 ? kSlotsPerSmMax : 2);
+    size_t slots = (size_t)sm_count() * attn_ctas_per_sm(D);
     if (slots > tiles) slots = tiles;
     if (B <= kSchedRows && 2 * slots > items) items = 2 * slots;
     return counters_bytes(B, NKV, nqt) + items * 16 * 2 * sizeof(float) + items * 16 * D * sizeof(float);
@@ -803,7 +806,7 @@ static cudaError_t launch_attn_instance(AttnParams& p, void* records, cudaStream
     int slots = 0;
     if (sched) {
         slots = attn_slots<D>();
-        const int most = sm_count() * (D <= 64 ? kSlotsPerSmMax : 2);
+        const int most = sm_count() * attn_ctas_per_sm(D);
         if (slots > most) slots = most;
         const long long tiles = (long long)p.B * p.NKV * p.nqt * ((p.S + kTileKeys - 1) / kTileKeys);
         if (slots > tiles) slots = (int)tiles;

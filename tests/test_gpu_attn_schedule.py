@@ -61,6 +61,25 @@ def test_ragged_attention(B, H, NKV, S, D, low):
         assert ((outs[0][b, :, 0].double() - want).norm() / want.norm()).item() < 6e-3, (b, n)
 
 
+def _ctas(B, H, NKV, S, D, lens):
+    """CTAs that a call runs on: one trace record each."""
+    Q, out = (torch.zeros(B, H, 1, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    K, V = (torch.zeros(B, NKV, S, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    lib = _lib.load()
+    ws = torch.zeros(lib.ezb_attn_decode_workspace_bytes(B, H, NKV, S, D), dtype=torch.uint8, device="cuda")
+    records = torch.zeros(4096 * 6, dtype=torch.int64, device="cuda")
+    cursor = torch.zeros(1, dtype=torch.int32, device="cuda")
+    try:
+        _lib.check(lib.ezb_trace_enable(records.data_ptr(), cursor.data_ptr(), 4096))
+        _lib.check(lib.ezb_attn_decode(Q.data_ptr(), K.data_ptr(), V.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel(), B, H, NKV, S, D,
+                                       None if lens is None else lens.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+    finally:
+        _lib.check(lib.ezb_trace_enable(None, None, 0))
+    assert _lib.device_status() == 0
+    return cursor.item()
+
+
 @pytest.mark.parametrize("B,H,NKV,S,D,ctas", [
     (64, 32, 8, 100, 128, 64 * 8),  # a row is one split: one CTA per (row, kv head)
     (128, 32, 8, 384, 128, 128 * 8),  # more groups than the fixed grid cuts
@@ -76,18 +95,13 @@ def test_which_shapes_are_balanced(B, H, NKV, S, D, ctas):
         ctas = torch.cuda.get_device_properties(0).multi_processor_count * (2 if D == 128 else 3)
     rng = random.Random(B)
     lens = torch.tensor([rng.randint(S // 8, S) for _ in range(B)], dtype=torch.int32, device="cuda")
-    Q, out = (torch.zeros(B, H, 1, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
-    K, V = (torch.zeros(B, NKV, S, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
-    lib = _lib.load()
-    ws = torch.zeros(lib.ezb_attn_decode_workspace_bytes(B, H, NKV, S, D), dtype=torch.uint8, device="cuda")
-    records = torch.zeros(4096 * 6, dtype=torch.int64, device="cuda")
-    cursor = torch.zeros(1, dtype=torch.int32, device="cuda")
-    try:
-        _lib.check(lib.ezb_trace_enable(records.data_ptr(), cursor.data_ptr(), 4096))
-        _lib.check(lib.ezb_attn_decode(Q.data_ptr(), K.data_ptr(), V.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel(), B, H, NKV, S, D,
-                                       lens.data_ptr(), torch.cuda.current_stream().cuda_stream))
-        torch.cuda.synchronize()
-    finally:
-        _lib.check(lib.ezb_trace_enable(None, None, 0))
-    assert cursor.item() == ctas
-    assert _lib.device_status() == 0
+    assert _ctas(B, H, NKV, S, D, lens) == ctas
+
+
+@pytest.mark.parametrize("D,per_sm", [(64, 3), (128, 2)])
+@pytest.mark.parametrize("B,S", [(1, 8192), (5, 4096), (8, 8192), (16, 1024), (24, 2048), (32, 512)])
+def test_rows_of_one_length_run_in_one_wave(B, S, D, per_sm):
+    """No more CTAs than are resident together (160 registers a thread leave room for three at head_dim 64, the ring for two
+    at 128): a second, partly filled wave costs a whole pass over a split."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert B * 8 <= _ctas(B, 32, 8, S, D, None) <= sms * per_sm
