@@ -140,6 +140,7 @@ static constexpr int kGroupUnits = 3;
 struct AttnSchedule {
     int end[kSchedRows];    // units (pieces or tiles) up to and including row b, over all its groups
     int tiles[kSchedRows];  // tiles of row b
+    int len[kSchedRows];    // valid keys of row b
     int lead;               // units without a tile in front of each group
     int chunk;              // > 0: chunks
     int whole;
@@ -191,9 +192,10 @@ __global__ void __launch_bounds__(kAttnThreads, attn_ctas_per_sm(D)) attn_decode
                 const int b = lane + 32 * i;
                 t[i] = 0;
                 if (32 * i >= p.B) continue;
-                t[i] = b < p.B ? max(1, (row_len(b) + kTileKeys - 1) / kTileKeys) : 0;  // an empty row writes zeros
+                const int len = b < p.B ? row_len(b) : 0;
+                t[i] = b < p.B ? max(1, (len + kTileKeys - 1) / kTileKeys) : 0;  // an empty row writes zeros
                 sum += t[i];
-                if (b < p.B) sched->tiles[b] = t[i];
+                if (b < p.B) sched->tiles[b] = t[i], sched->len[b] = len;
             }
             const int total = warp_sum_int(sum) * heads;
             const int even = max(p.min_tiles, (int)((total + gridDim.x - 1) / gridDim.x));
@@ -288,16 +290,15 @@ __global__ void __launch_bounds__(kAttnThreads, attn_ctas_per_sm(D)) attn_decode
                 skip_lead();
             }
             const int gi = rem / per;
-            sg.kvh = gi / p.nqt, sg.qt = gi % p.nqt, sg.rec_step = 2;
+            sg.kvh = gi / p.nqt, sg.qt = gi % p.nqt, sg.rec_step = 2, sg.len = sched->len[sg.b];
         } else {
             sg.part = blockIdx.x % p.nchunks, sg.nparts = p.nchunks, sg.qt = blockIdx.x / p.nchunks;
-            sg.kvh = blockIdx.y, sg.b = blockIdx.z;
-            const int ct = p.chunk / kTileKeys, all = (row_len(sg.b) + kTileKeys - 1) / kTileKeys;
+            sg.kvh = blockIdx.y, sg.b = blockIdx.z, sg.len = row_len(sg.b);
+            const int ct = p.chunk / kTileKeys, all = (sg.len + kTileKeys - 1) / kTileKeys;
             sg.t0 = min(all, sg.part * ct), sg.t1 = min(all, sg.t0 + ct);
             sg.rec0 = (((long long)sg.b * p.NKV + sg.kvh) * p.nqt + sg.qt) * p.nchunks, sg.rec1 = sg.rec0 + 1, sg.rec_step = 1;
             u0 = u1;
         }
-        sg.len = row_len(sg.b);
         return sg;
     };
     // Row (in units of D elements) of key `key` of a segment's (batch row, kv head) in the cache.
