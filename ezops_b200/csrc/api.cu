@@ -905,14 +905,13 @@ int ezb_tp_allreduce_f32(void* buf, void* const* comm_bases_host, int world, int
     return EZB_OK;
 }
 
-static int check_tp_fused_shape(int B, int H, int I_local, int NH_local, int NKV_local, int D) {
+static int check_tp_fused_shape(int B, int H, int I_local, int Q_local) {
     // every projection must run a kernel that knows the exchange: the small-batch kernel, or (batch >= 2)
     // the tensor-core kernel with the row kernel in front
-    auto covered = [&](int K, int N, bool pair) {
+    auto covered = [&](int K) {
         return gemv_small_batch_eligible(B, K) || (tuning(EZB_TUNE_TC) != 0 && gemm_tc_supported(B, K));
     };
-    EZB_REQUIRE_SHAPE(covered(H, (NH_local + 2 * NKV_local) * D, false) && covered(NH_local * D, H, false) &&
-                          covered(H, I_local, true) && covered(I_local, H, false),
+    EZB_REQUIRE_SHAPE(covered(H) && covered(Q_local) && covered(I_local),
                       "no kernel with the fused exchange covers this batch and these sizes");
     return EZB_OK;
 }
@@ -1029,7 +1028,7 @@ int ezb_qwen3_decode_layer_tp_fused(const void* hidden, void* K_cache, void* V_c
     TpLink base;
     if (int rc = make_tp_link(base, comm_bases_host, world, rank, B, H)) return rc;
     if (int rc = check_layer_args(B, S, H, I_local, NH_local, NKV_local, D)) return rc;
-    if (int rc = check_tp_fused_shape(B, H, I_local, NH_local, NKV_local, D)) return rc;
+    if (int rc = check_tp_fused_shape(B, H, I_local, NH_local * D)) return rc;
     EZB_REQUIRE(aligned16(hidden) && aligned16(K_cache) && aligned16(V_cache) && aligned16(Wqkv_local) &&
                     aligned16(Wo_local) && aligned16(Wgu_local) && aligned16(Wd_local) && aligned16(out),
                 "pointers must be 16-byte aligned");
@@ -1095,7 +1094,7 @@ int ezb_qwen3_decode_stack_tp_fused(const void* hidden, void* out, const ezb_lay
     TpLink base;
     if (int rc = make_tp_link(base, comm_bases_host, world, rank, B, H)) return rc;
     if (int rc = check_layer_args(B, S, H, I_local, NH_local, NKV_local, D)) return rc;
-    if (int rc = check_tp_fused_shape(B, H, I_local, NH_local, NKV_local, D)) return rc;
+    if (int rc = check_tp_fused_shape(B, H, I_local, NH_local * D)) return rc;
     EZB_REQUIRE(aligned16(hidden) && aligned16(out) && aligned16(rope_cos) && aligned16(rope_sin), "pointers must be 16-byte aligned");
     for (int l = 0; l < n_layers; ++l) {
         const ezb_layer_t& L = layers_local[l];

@@ -61,7 +61,9 @@ static constexpr long long kWaitLimitCycles = 2000000000LL;
 // consumers poll slot w of rank w's buffer with peer loads.  Measured on two GPUs (us per layer,
 // Qwen3-8B batch 32 KV 4096 | Qwen3-32B batch 64 KV 8192): NCCL all-reduce between the parts 162 | 345,
 // push 168 | 408, pull 200 | 433 - measured with a tensor-core kernel in which only the 32-40 CTAs that finished a tile
-// stored, 32-64 KB each (16-22 us); at batch <= 8 (every CTA stores a few values) push is the fast one.
+// stored, 32-64 KB each (16-22 us); with the small-batch kernel, up to 8 rows (every CTA stores a few values), push was
+// the fast one.  From 2 rows on the tensor-core kernel pushes now, where every CTA finishes columns of every tile; that form
+// has not been timed over NVLink.
 // ---------------------------------------------------------------------------
 struct TpLink {
     int world;  // 0: no fused exchange

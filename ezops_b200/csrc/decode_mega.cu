@@ -1119,6 +1119,7 @@ static bool mega_plan(const MegaArgs& a, MegaPlan& pl) {
     // hidden units fills half of its 64 KB stages, and the ring of three holds 96 KB.  Pieces of its own row length keep
     // the ring full of useful bytes (2B layer, KV 1024: 40.5 -> 38.2 us).  Shorter rows keep the longer pieces of the
     // other phases: cutting those to 1024 made the 0.6B layer 1..3 us slower (27.4 -> 28.4, KV 4096 30.2 -> 33.2).
+    // Only models of 1024, 2048, 4096 and 5120 hidden units have been measured; the lines between them are not.
     const int cap_kc = (a.H > 1024 && a.H <= 2048) ? 2048 : 4096;
     auto kc_of = [cap_kc](int K) { return K < cap_kc ? K : cap_kc; };
     pl.grid = grid;

@@ -206,7 +206,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 // Measured: Qwen3-8B layer, batch 32, KV 4096 187.9 -> 168.0 us; eight 2B layers, batch 13, paged 680 -> 488 us.
 // A norm in front of a projection is left to its epilogue (ssq_in): the kernel that produced the rows has written their
 // sums of squares and the rows times the norm weight, so no row kernel runs between two projections (3..6 us each; the
-// 2B layers above 488 -> 438 us, 28 layers of 0.6B at batch 4 928 -> 858 us).
+// 2B layers above 488 -> 438 us, 28 layers of 0.6B at batch 4 1008 -> 858 us).
 // LINK: the instance whose epilogue pushes its fp32 results into the peers' inboxes (see TpLink).
 template <int NB, bool LINK>
 __global__ void __launch_bounds__(kTcThreads, 2)

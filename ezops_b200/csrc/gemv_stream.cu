@@ -25,7 +25,8 @@
 // Every mbarrier wait is bounded (see mbar_wait_bounded).
 //
 // Two kernels share this structure:
-//   gemv_rows8_kernel   batch <= 8 with the activations resident: the weights are
+//   gemv_rows8_kernel   batch 1 (up to 8 rows where the tensor cores are not used,
+//                       see launch_gemv) with the activations resident: the weights are
 //                       the 8-wide B operand, so a stage is 8 whole weight rows
 //                       (up to 4096 elements = 8 KB per bulk copy, the size at
 //                       which the TMA unit reaches its streaming rate) and the
@@ -515,7 +516,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_stream_kernel(const Gemv
 
 
 // ---------------------------------------------------------------------------
-// Small-batch kernel (batch <= 8, activations resident).
+// Small-batch kernel (one row; it takes up to 8; activations resident).
 //
 // A stage holds 8 weight rows (4 gate + 4 up rows in PAIR mode) of up to 4096
 // elements each, one bulk copy per row.  ldmatrix.x4 on 8 rows x 32 k gives the
@@ -735,8 +736,6 @@ static int pick_nt(int B) { return B <= 8 ? 1 : (B <= 16 ? 2 : (B <= 32 ? 4 : 8)
 
 // Resident activations are worth it while they leave room for a useful ring.
 static bool x_fits_resident(int B, int K) { return (size_t)B * (K + 8) * 2 <= 72 * 1024 && B <= 8; }
-
-bool gemv_needs_scratch(int B, int K) { return !x_fits_resident(B, K); }
 
 
 PrefetchPlan prefetch_plan_rows(const bf16* W0, const bf16* W1, int N, int K, int cap_rows, int skip_rows) {

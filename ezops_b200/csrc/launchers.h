@@ -52,8 +52,8 @@ struct GemvArgs {
     long long ldres = 0;
     void* out = nullptr;  // [B, ldout] bf16 (fp32 for EPI_STORE_F32)
     long long ldout = 0;
-    bf16* xn_scratch = nullptr;  // [B, K] bf16: needed when the prologue cannot be fused (see gemv_needs_scratch)
-    PrefetchList next = {};  // what the following kernels stream first (optional)
+    bf16* xn_scratch = nullptr;  // [B, K] bf16: needed when the prologue cannot be fused (more than 8 rows, or the tensor cores)
+    PrefetchList next = {};  // what the following kernels stream first (optional; the tensor-core kernel pulls nothing ahead)
     int trace_id = 0;  // label in timeline traces
     bool allow_tc = false;  // batch >= 2: the tensor-core path may be taken
     // RMSNorm of this projection's result (EPI_RESIDUAL, EPI_PUSH_F32) or of its input (PRO_SCALED, PRO_ADD_RMSNORM
@@ -64,9 +64,9 @@ struct GemvArgs {
     TcTiling* tiling = nullptr;
     const bf16* next_norm_w = nullptr;
     bf16* xw_out = nullptr;
-    TpLink link = {0, 0, {}, {}, 0, -1, -1, -1};  // fused tensor-parallel exchange (small-batch kernel only)
+    TpLink link = {0, 0, {}, {}, 0, -1, -1, -1};  // fused tensor-parallel exchange (see launch_gemv for the kernels that have it)
 };
-bool gemv_small_batch_eligible(int B, int K);  // true when launch_gemv would run the small-batch kernel
+bool gemv_small_batch_eligible(int B, int K);  // the small-batch kernel takes these sizes (launch_gemv prefers the tensor cores if allowed)
 
 // Tensor-core (tcgen05) path for batched projections, see gemm_tc.cu.
 bool gemm_tc_supported(int B, int K);
@@ -77,10 +77,6 @@ cudaError_t launch_gemm_tc(const GemvArgs& a, const bf16* x, long long ldx, cuda
 PrefetchPlan prefetch_plan_rows(const bf16* W0, const bf16* W1, int N, int K, int cap_rows, int skip_rows = 0);  // a GEMV's weight rows
 PrefetchPlan prefetch_plan_flat(const void* a, const void* b, size_t bytes_each);            // whole regions
 
-// True when the activation block is too large to stay resident in shared memory
-// next to the weight ring, so a prologue has to run as a kernel of its own
-// writing to xn_scratch.
-bool gemv_needs_scratch(int B, int K);
 cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream);
 
 // -------------------------------------------------------------- row prep ---

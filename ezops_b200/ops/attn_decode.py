@@ -8,7 +8,9 @@ class opts into grouped-query attention with the class attribute
 
 Extension over the reference (one shared ``seq_len``): ``seq_lens`` gives one
 valid length per sequence, 1 <= len <= seq_len; keys past a row's length are
-not attended to (and not read).
+not attended to (and not read).  The order in which a row's keys are summed may
+depend on the lengths of all rows, so a sequence's result next to other sequences
+agrees within rounding, not bit for bit; equal calls give equal bits.
 """
 
 from __future__ import annotations

@@ -56,11 +56,11 @@ typedef struct CUstream_st* ezb_stream_t; /* same type as cudaStream_t */
 #define EZB_TUNE_GEMV_PREFETCH 2    /* weight stages requested before the dependency wait (0 = all; default 1) */
 #define EZB_TUNE_GEMV_CTAS_PER_SM 3 /* persistent CTAs per SM of the weight-streaming kernel            */
 #define EZB_TUNE_ATTN_MIN_CHUNK 4   /* smallest KV split, in keys (multiple of 64)                      */
-#define EZB_TUNE_ATTN_WAVES 5       /* rows of different lengths: 0 (default) = dealt out by their real lengths; n > 0 = n KV splits per SM on the grid of the longest row */
+#define EZB_TUNE_ATTN_WAVES 5       /* rows of different lengths: 0 (default) = dealt out by their real lengths where that is faster; n > 0 = n KV splits per SM on the grid of the longest row */
 #define EZB_TUNE_GEMV_KC 6          /* k-chunk length of a weight stage (0 = automatic)                 */
-#define EZB_TUNE_GEMV_ROWS8 7       /* 1: batch <= 8 uses the whole-row small-batch kernel (default 1)   */
+#define EZB_TUNE_GEMV_ROWS8 7       /* 1: small batches that do not run on the tensor cores use the whole-row kernel (default 1): one row, 2 to 4 rows of a stand-alone projection with few outputs, and up to 8 rows with EZB_TUNE_TC 0 */
 #define EZB_TUNE_PDL_ACROSS_CALLS 8 /* 1: the first kernel of a call may also start early (default 0)    */
-#define EZB_TUNE_L2_PREFETCH 9      /* 1: kernels of a chain pull the next kernel's first weights into L2 (default 1) */
+#define EZB_TUNE_L2_PREFETCH 9      /* 1: kernels of a chain pull the next kernel's first weights into L2 (default 1); from 2 rows on only the attention kernel does */
 #define EZB_TUNE_L2_PREFETCH_KB 10  /* KB per CTA of a following large weight pulled ahead (default 192)                 */
 #define EZB_TUNE_GEMV_WINDOW 11     /* stages that may be requested but not landed, small-batch kernel (0 = ring depth) */
 #define EZB_TUNE_L2_PREFETCH_ATTN_KB 12 /* KB per CTA of the gate/up weights that the attention kernel pulls ahead (default 0) */
@@ -107,10 +107,10 @@ int ezb_gemv_bf16(const void* x, const void* W, void* y, int N, int K, ezb_strea
 /* Batched form of the same kernel: Y[b, :] = W[N,K] . X[b, :] for b < B <= 64,
  * X [B,K], Y [B,N]; the weight is still streamed once for the whole batch.
  * (The reference op is batch 1 only; its fused ops hold the batched
- * projections, e.g. ezops/ops/qwen3_dense_decode.py:157.)  For B >= 2 the
- * workspace of ezb_gemv_workspace_bytes() is required (zero-filled once): larger
- * batches run on the tensor cores with a split over K that parks partial tiles
- * there. */
+ * projections, e.g. ezops/ops/qwen3_dense_decode.py:157.)  For B >= 2 a
+ * workspace of ezb_gemv_workspace_bytes() is required by contract, although no
+ * kernel behind this entry uses it at present (the parts of a split over K meet
+ * in shared memory). */
 size_t ezb_gemv_workspace_bytes(int B, int N, int K);
 int ezb_gemv_batched_bf16(const void* X, const void* W, void* Y, void* workspace, size_t workspace_bytes, int B, int N,
                           int K, ezb_stream_t stream);
@@ -146,7 +146,12 @@ int ezb_qk_norm_rope(const void* q, const void* k, const void* v, const void* qw
  * flash_decode_tilelang_gqa* kernels (ezops/kernels/attn_decode/attn_decode_tl.py:25-657)
  * behind AttnDecodeOp.forward (ezops/ops/attn_decode.py:55-56).
  * Q,Out [B,H,1,D]; K,V [B,NKV,S,D]; seq_lens_or_null int32[B] (1 <= len <= S).
- * D in {64, 128}; H % NKV == 0. */
+ * D in {64, 128}; H % NKV == 0.
+ * Calls with the same sizes and lengths give the same bits.  How a row is cut,
+ * and with it the order of its sums, may depend on the batch size and, with
+ * seq_lens, on the lengths of the OTHER rows: the same sequence next to other
+ * sequences agrees within rounding only.  The same holds for the layer and stack
+ * entries. */
 size_t ezb_attn_decode_workspace_bytes(int B, int H, int NKV, int S, int D);
 int ezb_attn_decode(const void* Q, const void* K, const void* V, void* Out, void* workspace, size_t workspace_bytes,
                     int B, int H, int NKV, int S, int D, const int* seq_lens_or_null, ezb_stream_t stream);

@@ -26,8 +26,7 @@ def main() -> int:
     dist.init_process_group("nccl", device_id=torch.device("cuda", local))
     ok = True
     # batch 1: the rank-local layer and both exchanges in one persistent kernel (and, with that switched off, in the
-    # small-batch kernels); batch 3: gather and push inside the small-batch kernel; batch 16: row kernel + tensor-core
-    # kernel; the last case is the benchmark's tensor-parallel configuration (Qwen3-32B shapes, batch 64) at a shorter cache
+    # small-batch kernels); batch 3 and 16: the row kernel gathers, the tensor-core kernel pushes; the last case is the benchmark's tensor-parallel configuration (Qwen3-32B shapes, batch 64) at a shorter cache
     for sh, B, S in [(wl.QWEN3_VL_2B, 1, 700), (wl.QWEN3_8B, 1, 2100), (wl.QWEN3_8B, 3, 1025), (wl.QWEN3_VL_2B, 16, 400),
                      (wl.QWEN3_32B, 64, 1536)]:
         hidden, K0, V0, Wqkv, Wo, Wgu, Wd = wl.decode_layer_inputs(sh, B, S)
