@@ -825,8 +825,13 @@ static cudaError_t launch_attn_instance(AttnParams& p, void* records, cudaStream
         // Head dim 64: a new group costs as much as at 128 but its tiles cost half, so the schedule gains only where groups
         // are few and long (11 rows of 512..4096 keys 17.3 us on the grid, 14.8 by schedule) and loses elsewhere (64 rows of
         // 64..512 keys 15.2 and 19.5).  Over 2000 shapes this rule is 11..14 % faster than the schedule wherever something
-        // is cut, the grid everywhere 10..12 %.
-        else if (D <= 64 && (2 * groups > slots || tiles <= 4LL * slots)) sched = false;
+        // is cut, the grid everywhere 10..12 %.  Few and short groups leave the chip half empty anyway: one wave of splits
+        // as for rows of one length (1 row of 8192 keys at most: 12.8 us in more, shorter splits, 10.6 so).
+        else if (D <= 64 && (2 * groups > slots || tiles <= 4LL * slots)) {
+            sched = false;
+            if (2 * groups <= slots) p.chunk = max(p.chunk, attn_chunk_keys(p.B, p.NKV, p.S, false, D));
+            p.nchunks = (p.S + p.chunk - 1) / p.chunk;
+        }
     }
     const size_t items = sched ? 2 * (size_t)slots : (size_t)p.B * p.NKV * p.nqt * p.nchunks;
     p.part_ml = static_cast<float*>(records);

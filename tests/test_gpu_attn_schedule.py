@@ -21,6 +21,8 @@ CASES = [
     (24, 32, 8, 3000, 128, 100),  # ranges
     (24, 8, 8, 4096, 64, 1),  # ranges, head_dim 64
     (40, 8, 8, 4096, 64, 1),  # fixed grid, head_dim 64
+    (1, 32, 8, 8192, 64, 8000),  # few and short groups, head_dim 64: one wave of splits, more than the fast fold takes
+    (5, 16, 16, 900, 64, 1),
     (128, 16, 8, 257, 128, 1),  # the most rows the schedule covers
     (129, 8, 8, 257, 128, 1),  # one more
     (2, 64, 2, 3000, 128, 10),  # two query tiles per kv head
@@ -84,6 +86,7 @@ def _ctas(B, H, NKV, S, D, lens):
     (64, 32, 8, 100, 128, 64 * 8),  # a row is one split: one CTA per (row, kv head)
     (128, 32, 8, 384, 128, 128 * 8),  # more groups than the fixed grid cuts
     (64, 32, 8, 512, 64, 64 * 8 * 2),  # head_dim 64, many short groups: two splits each
+    (1, 32, 8, 8192, 64, 8 * 43),  # head_dim 64, few and short groups: splits of 192 keys, one wave
     (4, 16, 8, 1024, 128, 4 * 8 * 8),  # the smallest splits of full rows fit one wave
     (32, 32, 8, 8192, 128, None),  # balanced: two CTAs per SM
     (11, 32, 8, 4096, 64, None),  # head_dim 64, few long groups: three
