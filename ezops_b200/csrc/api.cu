@@ -935,7 +935,7 @@ static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_
     const bf16* hid = gather_prev ? layer_in : x_prev;
     {   // QKV projection (norm prologue; gathers the previous layer's second sum when there is one)
         GemvArgs g;
-        g.allow_tc = B >= 2, g.xn_scratch = w.xn;
+        g.allow_tc = B >= 2, g.xn_scratch = w.xn, g.behind_gather = true;
         g.W0 = Wqkv, g.ldw = H, g.N = rows, g.K = H, g.B = B;
         g.x = x_prev, g.ldx = H;
         g.norm_w = ex.input_norm_w;
@@ -968,7 +968,7 @@ static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_
     }
     {   // o_proj: partial -> inbox 0 of every rank; also opens the next epoch of inbox 1
         GemvArgs g;
-        g.allow_tc = B >= 2, g.xn_scratch = w.xn;
+        g.allow_tc = B >= 2, g.xn_scratch = w.xn, g.behind_gather = true;
         g.W0 = Wo, g.ldw = Q, g.N = H, g.K = Q, g.B = B;
         g.x = w.attn_out, g.ldx = Q;
         g.epilogue = EPI_PUSH_F32, g.ldout = H;
@@ -980,7 +980,7 @@ static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_
     }
     {   // gate/up: x2 = layer input + sum(inbox 0), norm, SwiGLU
         GemvArgs g;
-        g.allow_tc = B >= 2, g.xn_scratch = w.xn;
+        g.allow_tc = B >= 2, g.xn_scratch = w.xn, g.behind_gather = true;
         g.W0 = wgu, g.W1 = wgu + (size_t)I_local * H, g.ldw = H, g.N = I_local, g.K = H, g.B = B;
         g.x = hid, g.ldx = H;
         g.x_sum_out = x2_out, g.ldsum = H;
@@ -995,7 +995,7 @@ static int run_layer_tp_fused(const bf16* x_prev, bool gather_prev, bf16* layer_
     }
     {   // down: partial -> inbox 1 of every rank; opens the next epoch of inbox 0
         GemvArgs g;
-        g.allow_tc = B >= 2, g.xn_scratch = w.xn;
+        g.allow_tc = B >= 2, g.xn_scratch = w.xn, g.behind_gather = true;
         g.W0 = Wd, g.ldw = I_local, g.N = H, g.K = I_local, g.B = B;
         g.x = w.h, g.ldx = I_local;
         g.epilogue = EPI_PUSH_F32, g.ldout = H;

@@ -18,7 +18,7 @@
 //     to the clusters that fit on the chip (tc_plan below);
 //   * a CTA takes at most half of an SM (shared memory, registers, tensor memory), so that the next kernel of a chain
 //     can be resident while this one drains and already has its weight ring in flight when its input is complete.
-//   * the LINK instance pushes its fp32 results into the tensor-parallel peers' inboxes (see TpLink).
+//   * the LINK instance serves the fused tensor-parallel exchange (see TpLink).
 // Every mbarrier wait is bounded; on a time-out the CTA records a fault, stops issuing work, waits (bounded) for
 // copies in flight, frees its tensor memory and returns.
 #include <cuda.h>
@@ -207,7 +207,8 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 // A norm in front of a projection is left to its epilogue (ssq_in): the kernel that produced the rows has written their
 // sums of squares and the rows times the norm weight, so no row kernel runs between two projections (3..6 us each; the
 // 2B layers above 488 -> 438 us, 28 layers of 0.6B at batch 4 1008 -> 858 us).
-// LINK: the instance whose epilogue pushes its fp32 results into the peers' inboxes (see TpLink).
+// LINK: the instance for chains with the fused exchange: its epilogue can push fp32 results into the peers' inboxes (see
+// TpLink), and its waits start behind the gather of the kernel in front.
 template <int NB, bool LINK>
 __global__ void __launch_bounds__(kTcThreads, 2)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant__ CUtensorMap mapW1,
@@ -329,10 +330,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapW0, const __grid_constant_
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         if (elect_one()) {
-            // A stage is full only with the X block that the producer requests behind its own dependency wait.  Waiting
-            // here too keeps the time that the kernel in front takes - a gather may wait for its peers for seconds, and
-            // has released this kernel before - out of the budget of the waits below.
-            pdl_wait();
+            // A stage is full only with the X block that the producer requests behind its own dependency wait.  Behind a
+            // gather, which may wait for its peers for seconds and has released this kernel before, waiting here too keeps
+            // that time out of the budget of the waits below.  (Elsewhere it only costs, even as a branch not taken: 30 ns
+            // a projection.)
+            if (LINK) pdl_wait();
             int stage = 0;
             uint32_t full_parity = 0;
             for (int i = 0; i < my_tiles && !(*abort_flag); ++i) {
@@ -767,7 +769,7 @@ cudaError_t launch_gemm_tc(const GemvArgs& a, const bf16* x, long long ldx, cuda
     p.link = a.link;
     if (a.link.world > 0 && (a.link.gather_inbox >= 0 || pair)) return cudaErrorNotSupported;  // only the push side lives here
     const int NB = tc_batch_tile(a.B);
-    if (a.link.world > 0) {
+    if (a.link.world > 0 || a.behind_gather) {
         switch (NB) {
             case 16: return launch_tc_instance<16, true>(a, x, ldx, p, stream);
             case 32: return launch_tc_instance<32, true>(a, x, ldx, p, stream);

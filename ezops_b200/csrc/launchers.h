@@ -64,6 +64,7 @@ struct GemvArgs {
     TcTiling* tiling = nullptr;
     const bf16* next_norm_w = nullptr;
     bf16* xw_out = nullptr;
+    bool behind_gather = false;  // kernels in front of this one may wait for tensor-parallel peers
     TpLink link = {0, 0, {}, {}, 0, -1, -1, -1};  // fused tensor-parallel exchange (see launch_gemv for the kernels that have it)
 };
 bool gemv_small_batch_eligible(int B, int K);  // the small-batch kernel takes these sizes (launch_gemv prefers the tensor cores if allowed)
