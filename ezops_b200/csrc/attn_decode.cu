@@ -167,8 +167,8 @@ __global__ void __launch_bounds__(kAttnThreads, attn_ctas_per_sm(D)) attn_decode
     const int g4 = lane >> 2, t4 = lane & 3;
     const int G = p.G;
     const int cta = SCHED ? (int)blockIdx.x : (int)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
-    // Lengths and page ids may be read before the dependency wait (`early`): through L2, since a line that an earlier
-    // kernel left in this SM's L1 is only known to be dropped behind that wait.
+    // Lengths and the first page ids may be read before the dependency wait (`early`): through L2, since a line that an
+    // earlier kernel left in this SM's L1 is only known to be dropped behind that wait.
     auto row_len = [&](int b) { return p.seq_lens ? max(p.fuse_new_token ? 1 : 0, min(p.S, __ldcg(p.seq_lens + b))) : p.S; };
 
     unsigned long long* trec = (tid == 0) ? trace_open(p.trace, 9u, cta) : nullptr;
@@ -304,10 +304,11 @@ __global__ void __launch_bounds__(kAttnThreads, attn_ctas_per_sm(D)) attn_decode
     // Row (in units of D elements) of key `key` of a segment's (batch row, kv head) in the cache.
     // A page id outside the pools (a stale or "unallocated" -1 entry) sets ok = false and records a fault; the
     // caller then touches no memory for that key.
-    auto cache_row = [&](const AttnSegment& sg, int key, bool& ok) -> long long {
+    auto cache_row = [&](const AttnSegment& sg, int key, bool& ok, bool before_wait) -> long long {
         ok = true;
         if (!p.page_table) return ((long long)sg.b * p.NKV + sg.kvh) * p.S + key;
-        const long long page = __ldcg(p.page_table + (long long)sg.b * p.max_pages + (key >> p.page_shift));
+        const int* entry = p.page_table + (long long)sg.b * p.max_pages + (key >> p.page_shift);
+        const long long page = before_wait ? __ldcg(entry) : *entry;
         if (page < 0 || page >= p.num_pages) {
             report_fault(p.status, FAULT_PAGE_RANGE);
             ok = false;
@@ -336,7 +337,7 @@ __global__ void __launch_bounds__(kAttnThreads, attn_ctas_per_sm(D)) attn_decode
     // A segment's start-up window: norm weights and rotary rows (inputs of the call), then its first two tiles; always
     // three commit groups.  In decode-layer mode slot len-1 still holds stale data when its tile is requested; the CTA
     // that owns it overwrites that row in shared memory once the tile has landed (see the loop below).
-    auto open_segment = [&](const AttnSegment& sg, int ring) {
+    auto open_segment = [&](const AttnSegment& sg, int ring, bool before_wait) {
         static_assert(kAttnStages == 3, "two tiles ahead, one stage for the merge");
         if (p.fuse_new_token && tid < 4 * CPR) {
             const int which = tid / CPR, c = tid % CPR;
@@ -346,8 +347,8 @@ __global__ void __launch_bounds__(kAttnThreads, attn_ctas_per_sm(D)) attn_decode
         cp_async_commit();
         const int n = tiles_of(sg);
         bool ok0 = true, ok1 = true;
-        const long long r0 = n > 0 ? cache_row(sg, sg.t0 * kTileKeys, ok0) : 0;
-        const long long r1 = n > 1 ? cache_row(sg, (sg.t0 + 1) * kTileKeys, ok1) : 0;
+        const long long r0 = n > 0 ? cache_row(sg, sg.t0 * kTileKeys, ok0, before_wait) : 0;
+        const long long r1 = n > 1 ? cache_row(sg, (sg.t0 + 1) * kTileKeys, ok1, before_wait) : 0;
         if (n > 0) load_tile(sg, 0, ring % kAttnStages, r0, ok0);
         cp_async_commit();
         if (n > 1) load_tile(sg, 1, (ring + 1) % kAttnStages, r1, ok1);
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(kAttnThreads, attn_ctas_per_sm(D)) attn_decode
 
     int ring = 0;  // tiles of the segments before this one: tile t of a segment lives in stage (ring + t) % 3
     AttnSegment sg = take_segment();
-    open_segment(sg, ring);
+    open_segment(sg, ring, p.early);
     if (p.early) pdl_wait();
     trace_mark(trec, 3);
 
@@ -416,7 +417,7 @@ __global__ void __launch_bounds__(kAttnThreads, attn_ctas_per_sm(D)) attn_decode
                 // written to cache slot S-1 (nobody reads that slot from memory in this kernel)
                 if (owns_new_slot && warp < 2) {
                     bool slot_ok = true;
-                    const long long slot = cache_row(sg, new_slot, slot_ok) * D;
+                    const long long slot = cache_row(sg, new_slot, slot_ok, false) * D;
                     const bool write_slot = slot_ok && qt == 0;  // a bad page: the new k / v are not written anywhere
                     if (warp == 0) {
                         float x[D / 32];
@@ -460,14 +461,14 @@ __global__ void __launch_bounds__(kAttnThreads, attn_ctas_per_sm(D)) attn_decode
 
         // the cache row of the tile two ahead is looked up one iteration before its copy is issued
         bool ahead_ok = true;
-        long long ahead = ntiles > 2 ? cache_row(sg, c0 + 2 * kTileKeys, ahead_ok) : 0;
+        long long ahead = ntiles > 2 ? cache_row(sg, c0 + 2 * kTileKeys, ahead_ok, false) : 0;
         for (int t = 0; t < ntiles; ++t) {
             cp_async_wait<kAttnStages - 2>();
             __syncthreads();
             if (t == 0) trace_mark(trec, 4);
             if (t + 2 < ntiles) load_tile(sg, t + 2, (ring + t + 2) % kAttnStages, ahead, ahead_ok);
             cp_async_commit();
-            if (t + 3 < ntiles) ahead = cache_row(sg, c0 + (t + 3) * kTileKeys, ahead_ok);
+            if (t + 3 < ntiles) ahead = cache_row(sg, c0 + (t + 3) * kTileKeys, ahead_ok, false);
             if (owns_new_slot && t == ntiles - 1) {
                 // overwrite the stale row of slot S-1 in this tile with the new token's k and v
                 const int r = new_slot - (c0 + t * kTileKeys);
@@ -557,7 +558,7 @@ __global__ void __launch_bounds__(kAttnThreads, attn_ctas_per_sm(D)) attn_decode
         AttnSegment next = sg;
         if (more) {
             next = take_segment();
-            open_segment(next, ring);
+            open_segment(next, ring, false);
         }
         __syncthreads();
 
